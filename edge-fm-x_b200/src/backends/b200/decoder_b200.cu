@@ -697,7 +697,7 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
     while (first < n_entries) {
         std::vector<RowEntry> re;
         std::vector<int32_t> ids, row_entry;
-        std::vector<RowTile> tc, simt, ws;
+        std::vector<RowTile> tc, ws;
         std::vector<int32_t> short_rows;
         int n_ws = 0;
         struct Want { int32_t row; int64_t idx; uint32_t rng_step; };
@@ -708,11 +708,12 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
             const int n = std::min(en.n_tokens - done[e], c->max_s - rows);
             KvSlot& s = c->slots.at(en.slot);
             RowEntry r{rows, n, en.kv_offset + done[e], s.table, s.state_slot, 0};
-            const int idx = (int)re.size(), step = n >= kTcMinRows ? decoder_tc_tile_rows() : decoder_simt_tile_rows();
-            for (int i = 0; i < n; i += step) (n >= kTcMinRows ? tc : simt).push_back(RowTile{idx, i});
+            const int idx = (int)re.size();
             if (n < kTcMinRows)
                 for (int i = 0; i < n; ++i) short_rows.push_back(rows + i);
-            else if (m.ws_pages > 0) {
+            else
+                for (int i = 0; i < n; i += decoder_tc_tile_rows()) tc.push_back(RowTile{idx, i});
+            if (n >= kTcMinRows && m.ws_pages > 0) {
                 const int p0 = decoder_ws_page0(m, r.pos0), p1 = (r.pos0 + n - 1) / EFM_PAGE_TOKENS;
                 r.ws0 = (n_ws - p0) * EFM_PAGE_TOKENS;
                 n_ws += p1 - p0 + 1;
@@ -732,9 +733,9 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
         // late rows see the most keys; the kernel takes the last tiles first
         std::stable_sort(tc.begin(), tc.end(), [&](const RowTile& a, const RowTile& b) { return re[a.entry].pos0 + a.row < re[b.entry].pos0 + b.row; });
         // tiles of the tensor-core form go to the CUDA-core form in layers it does not take: list them in its units too
-        std::vector<RowTile> all_simt;
+        std::vector<RowTile> simt;
         for (size_t i = 0; i < re.size(); ++i)
-            for (int r = 0; r < re[i].n; r += decoder_simt_tile_rows()) all_simt.push_back(RowTile{(int32_t)i, r});
+            for (int r = 0; r < re[i].n && re[i].n >= kTcMinRows; r += decoder_simt_tile_rows()) simt.push_back(RowTile{(int32_t)i, r});
         std::vector<int32_t> pk;
         auto put = [&](const void* p, size_t words) {
             const size_t at = pk.size();
@@ -746,8 +747,7 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
         for (const Want& w : wants) want_rows.push_back(w.row);
         const size_t o_ids = put(ids.data(), ids.size()), o_re = put(re.data(), re.size() * sizeof(RowEntry) / 4),
                      o_row = put(row_entry.data(), row_entry.size()), o_tc = put(tc.data(), tc.size() * 2), o_simt = put(simt.data(), simt.size() * 2),
-                     o_all = put(all_simt.data(), all_simt.size() * 2), o_want = put(want_rows.data(), want_rows.size()),
-                     o_short = put(short_rows.data(), short_rows.size()), o_ws = put(ws.data(), ws.size() * 2);
+                     o_want = put(want_rows.data(), want_rows.size()), o_short = put(short_rows.data(), short_rows.size()), o_ws = put(ws.data(), ws.size() * 2);
         if (pk.size() > m.step_words) {
             EFM_CK(c, cudaStreamSynchronize(c->stream));
             EFM_CK(c, dev_alloc(c, &m.step_buf, pk.size() * 2, false));
@@ -767,8 +767,6 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
         tiles.n_tc = (int)tc.size();
         tiles.simt = reinterpret_cast<const RowTile*>(m.step_buf + o_simt);
         tiles.n_simt = (int)simt.size();
-        tiles.all = reinterpret_cast<const RowTile*>(m.step_buf + o_all);
-        tiles.n_all = (int)all_simt.size();
         tiles.short_rows = m.step_buf + o_short;
         tiles.n_short = (int)short_rows.size();
         tiles.ws_pages = reinterpret_cast<const RowTile*>(m.step_buf + o_ws);

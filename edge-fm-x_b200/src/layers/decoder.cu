@@ -223,6 +223,31 @@ void launch_attn_decode(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, con
     else rot ? launch_attn_decode_v<TC, 256, true>(L, p, cluster) : launch_attn_decode_v<TC, 256, false>(L, p, cluster);
 }
 
+// Rows of the short entries of a pass: `rows` lists them (null: all).
+template <typename T, int VM>
+void launch_attn_short_v(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const DecoderRun& run, const WindowAttnShape& s, const RowPlan& plan, const int32_t* rows, int n) {
+    DecoderModel& m = *c.decoder;
+    const int hb = (s.H / s.G + wd::kHeads - 1) / wd::kHeads;
+    int pages = m.d.cache_pages;
+    if (s.window > 0) pages = std::min(pages, (s.window + s.keep + kPageTokens - 1) / kPageTokens);
+    // A block per 64 visible keys, but no more blocks than stay resident at a time (4 a SM): further ones would only add merges.
+    int splits = 1;
+    while (splits < pages && splits < m.attn_cluster && (int64_t)2 * splits * s.G * hb * n <= 4 * c.num_sms) splits *= 2;
+    for (int r0 = 0; r0 < n; r0 += 32768) {                          // grid.z
+        L.cluster_x = splits;
+        L.launch(window_attention_short_kernel<T, VM>, dim3(splits, s.G * hb, std::min(n - r0, 32768)), dim3(wd::kThreads), sizeof(wd::Smem<VM>),
+                 static_cast<const T*>(m.q), static_cast<const T*>(run.k_pool), static_cast<const T*>(run.v_pool), static_cast<T*>(m.mix), l.mix_wp, s, plan,
+                 rows != nullptr ? rows + r0 : nullptr);
+    }
+}
+template <typename T>
+void launch_attn_short(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const DecoderRun& run, const WindowAttnShape& s, const RowPlan& plan, const int32_t* rows, int n) {
+    const int v = std::max(s.Dp, s.Vp);
+    if (v <= 64) launch_attn_short_v<T, 64>(c, L, l, run, s, plan, rows, n);
+    else if (v <= 128) launch_attn_short_v<T, 128>(c, L, l, run, s, plan, rows, n);
+    else launch_attn_short_v<T, 256>(c, L, l, run, s, plan, rows, n);
+}
+
 // ---- latent attention, absorbed form: a decode step, or rows of a pass ---------------------------------------------------
 // keys per tile, at most `most`, that the block's shared memory takes next to everything else
 int latent_tile(const LatentShape& s, int nh, int splits, int es, int most) {
@@ -813,20 +838,19 @@ void attention_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const D
             L.launch(window_attention_rows_kernel<TA, TA, TA>, dim3(n, s.H), dim3(256), wa::rows_smem_bytes(s.Dp, s.Vp), static_cast<const TA*>(m.q),
                      (const TA*)kp, (const TA*)vp, static_cast<TA*>(m.mix), l.mix_wp, s, plan, list);
     };
+    if (tiles.listed && tiles.n_short > 0) launch_attn_short<TA>(c, L, l, run, s, plan, tiles.short_rows, tiles.n_short);
+    if (!tiles.listed && plan.rows < kTcMinRows) {
+        launch_attn_short<TA>(c, L, l, run, s, plan, nullptr, plan.rows);
+        return;
+    }
     if constexpr (std::is_same<TA, __nv_bfloat16>::value) {
         if (decoder_layer_tc(m, l)) {
-            if (tiles.listed) {
-                launch_attention_tc(c, L, l, run, s, plan, tiles.tc, tiles.n_tc);
-                cuda_cores(tiles.simt, tiles.n_simt);
-                return;
-            }
-            if (plan.rows >= kTcMinRows) {
-                launch_attention_tc(c, L, l, run, s, plan, nullptr, (plan.rows + wt::BM - 1) / wt::BM);
-                return;
-            }
+            if (tiles.listed) launch_attention_tc(c, L, l, run, s, plan, tiles.tc, tiles.n_tc);
+            else launch_attention_tc(c, L, l, run, s, plan, nullptr, (plan.rows + wt::BM - 1) / wt::BM);
+            return;
         }
     }
-    cuda_cores(tiles.all, tiles.listed ? tiles.n_all : (plan.rows + wa::QT - 1) / wa::QT);
+    cuda_cores(tiles.simt, tiles.listed ? tiles.n_simt : (plan.rows + wa::QT - 1) / wa::QT);
 }
 
 template <typename TA>
@@ -1096,10 +1120,9 @@ namespace {
 template <typename K>
 cudaError_t smem_attr(K kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
 
-// widest cluster the decode attention kernel can be placed with
-template <typename TC, int VM, bool ROT, bool LIN>
-cudaError_t fit_cluster_v(int& width) {
-    const auto kernel = window_attention_decode_kernel<TC, VM, ROT, LIN>;
+// widest cluster the decode attention kernels can be placed with
+template <int VM, typename K>
+cudaError_t fit_cluster_v(K kernel, int& width) {
     cudaError_t e = smem_attr(kernel, sizeof(wd::Smem<VM>));
     if (e != cudaSuccess) return e;
     const bool wide = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
@@ -1124,8 +1147,9 @@ cudaError_t fit_cluster_v(int& width) {
 }
 template <typename TC, int VM, bool ROT>
 cudaError_t fit_cluster(int& width) {
-    const cudaError_t e = fit_cluster_v<TC, VM, ROT, false>(width);
-    return e == cudaSuccess ? fit_cluster_v<TC, VM, ROT, true>(width) : e;
+    cudaError_t e = fit_cluster_v<VM>(window_attention_decode_kernel<TC, VM, ROT, false>, width);
+    if (e == cudaSuccess) e = fit_cluster_v<VM>(window_attention_decode_kernel<TC, VM, ROT, true>, width);
+    return e == cudaSuccess && !ROT ? fit_cluster_v<VM>(window_attention_short_kernel<TC, VM>, width) : e;
 }
 }  // namespace
 

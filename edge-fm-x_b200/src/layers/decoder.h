@@ -138,13 +138,12 @@ struct DecoderModel {
 // One decode step of the bound slot (reads the device state); sample: run the sampler and advance the state.
 void decoder_decode_step(efm_b200_ctx& c, KvSlot& slot, Launcher& L, bool sample, bool want_logits);
 // One pass over rows [0, plan.rows) with ids on the device; the residual stream is left in c.resid.
-// Attention work lists of a batched pass (listed): tensor-core tiles of the long entries, CUDA-core tiles of the short
-// ones, and every row in CUDA-core tiles (layers the tensor-core form does not take).  Not listed: the single entry.
+// Attention work lists of a batched pass (listed): tensor-core tiles of the long entries, the same rows in CUDA-core tiles (layers
+// the tensor-core form does not take), and the rows of the short entries.  Not listed: the single entry.
 struct RowTiles {
-    const RowTile *tc = nullptr, *simt = nullptr, *all = nullptr;
-    int n_tc = 0, n_simt = 0, n_all = 0;
-    // latent attention: rows of the short entries (absorbed form); workspace pages of the long entries and those of them that
-    // hold earlier tokens (listed, or from ws_page0 on)
+    const RowTile *tc = nullptr, *simt = nullptr;
+    int n_tc = 0, n_simt = 0;
+    // latent attention: workspace pages of the long entries and those of them that hold earlier tokens (listed, or from ws_page0 on)
     const int32_t* short_rows = nullptr;
     const RowTile* ws_pages = nullptr;
     int n_short = 0, n_ws = 0, n_gather = 0, ws_page0 = 0;
@@ -153,7 +152,7 @@ struct RowTiles {
 void decoder_rows_pass(efm_b200_ctx& c, const RowPlan& plan, const int32_t* ids, const RowTiles& tiles, Launcher& L);
 // logits_rows[i] = head . norm(resid[rows[i]]), i < n <= max_want; rows on the device
 void decoder_rows_logits(efm_b200_ctx& c, const int32_t* rows, int n, Launcher& L);
-// Rows of one entry that share an attention block; entries shorter than kTcMinRows run on the CUDA-core form.
+// Rows of one entry that share an attention block; rows of entries shorter than kTcMinRows are walked one by one.
 constexpr int kTcMinRows = 16;
 int decoder_tc_tile_rows();
 int decoder_simt_tile_rows();

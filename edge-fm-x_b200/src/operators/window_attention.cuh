@@ -7,8 +7,9 @@
 // Dp / Vp (multiples of 64); a sequence's pages are listed in a page table.  TC = bf16 or fp32 (the all-32-bit mode).
 //
 //   qk_scatter_rows      many rows: per-head norms and rotation, q -> [T][H][Dp], k and v -> cache rows
-//   window_attention_rows many rows on the CUDA cores, fp32 throughout (32-bit mode, short portions, head sizes the
-//                        tensor-core form does not take)
+//   window_attention_rows many rows on the CUDA cores, fp32 throughout (32-bit mode, head sizes the tensor-core form does not take)
+//   window_attention_short rows of entries too short for the tensor-core form (decoded tokens of many sequences, short portions):
+//                        the walk of window_attention_decode for every row
 //   window_attention_decode one row: norms of q and k, cache append and split-key attention in one launch; the splits of
 //                        a kv head are the blocks of one cluster and merge through distributed shared memory
 #pragma once
@@ -372,8 +373,195 @@ template <> struct Row4<float> {
     __device__ __forceinline__ void get(float (&f)[4]) const { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
 };
 
-// grid (splits = cluster size, kv_heads * head blocks); the visible keys (kept first tokens, then the window) are numbered in
-// order and dealt out evenly, block `split` walks its share in tiles of 64.  VM: upper bound of Dp and Vp.  Further rows of
+// The keys of one row that a block walks.  The visible ones (kept first tokens, then the window) are numbered in order; key number n
+// stands at position n or, behind the kept ones, n + skip.  newest: the number of the key that is in shared memory instead of the
+// cache (-1: none).
+struct SplitKeys {
+    int pos, kept, skip, newest, begin, end;
+    __device__ __forceinline__ SplitKeys(const WindowAttnShape& s, int pos_, bool ok, int split, int n_splits) {
+        pos = pos_;
+        const int lo = s.window > 0 ? max(0, pos + 1 - s.window) : 0;
+        kept = s.window > 0 ? min(s.keep, lo) : 0;
+        skip = lo - kept;
+        const int n_vis = pos + 1 - skip, chunk = ok ? (n_vis + n_splits - 1) / n_splits : 0;
+        newest = n_vis - 1;
+        begin = split * chunk;
+        end = ok ? min(n_vis, begin + chunk) : begin;
+    }
+    __device__ __forceinline__ int position(int n) const { return n < kept ? n : n + skip; }
+};
+
+// Requests 64 keys from number j0 on, except the newest: 4 threads per key for the scores, 4 channels a thread for the sum.
+template <typename TC, int KC, int VK, class Row>
+__device__ __forceinline__ void window_load_tile(const WindowAttnShape& s, const SplitKeys& k, int j0, int g, const TC* k_pool, const TC* v_pool, Row&& pool_row,
+                                                 Row8<TC> (&kr)[KC], Row4<TC> (&vr)[VK]) {
+    const int tid = threadIdx.x, key = tid >> 2, part = tid & 3, tpr = s.Vp / 4, kg = wd::kThreads / tpr, dpart = tid % tpr, tg = tid / tpr;
+    const int j = j0 + key;
+    if (j < k.end && j != k.newest) {
+        const TC* src = k_pool + (pool_row(k.position(j)) * s.G + g) * s.Dp;
+#pragma unroll
+        for (int c = 0; c < KC; ++c)
+            if ((c * 4 + part) * 8 < s.Dp) kr[c].load(src + (c * 4 + part) * 8);
+    }
+    if (tg < kg) {
+#pragma unroll
+        for (int i = 0; i < VK; ++i) {
+            const int kk = tg + i * kg, jj = j0 + kk;
+            if (kk < kPageTokens && jj < k.end && jj != k.newest) vr[i].load(v_pool + (pool_row(k.position(jj)) * s.G + g) * s.Vp + dpart * 4);
+        }
+    }
+}
+
+// Scores, softmax and sum over a block's keys in tiles of 64 (the first one requested), then the merge over the cluster's blocks.
+// sm.q holds the heads' queries, sm.m / sm.l their empty sums; emit(head, channel, value) gets this block's share of the outputs.
+template <typename TC, int VM, int KC, int VK, class Load, class Cluster, class Token, class Gate, class Emit>
+__device__ __forceinline__ void window_split_walk(wd::Smem<VM>& sm, const WindowAttnShape& s, const SplitKeys& k, int h0, int nh, Row8<TC> (&kr)[KC], Row4<TC> (&vr)[VK],
+                                                  Load&& load_tile, Cluster& cl, Token& started, Gate&& gate_of, Emit&& emit) {
+    using namespace wd;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, split = blockIdx.x, n_splits = gridDim.x;
+    const int key = tid >> 2, part = tid & 3;                          // score phase
+    const int tpr = s.Vp / 4, kg = kThreads / tpr, dpart = tid % tpr, tg = tid / tpr;     // P.V phase: 4 channels per thread
+    const bool pv = tg < kg;
+    float acc[kHeads][4];
+#pragma unroll
+    for (int h = 0; h < kHeads; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[h][j] = 0.f;
+
+    for (int j0 = k.begin; j0 < k.end; j0 += kPageTokens) {
+        const int j = j0 + key;
+        const bool vis = j < k.end;
+        // ---- scores: 4 threads per key ----------------------------------------------------------------------------
+        float kf[KC][8];
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            const int d0 = (c * 4 + part) * 8;
+            if (d0 < s.Dp && j == k.newest) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) kf[c][i] = sm.knew[d0 + i];
+            } else {
+                kr[c].get(kf[c]);
+            }
+        }
+        for (int h = 0; h < nh; ++h) {
+            float d = 0.f;
+            if (vis) {
+#pragma unroll
+                for (int c = 0; c < KC; ++c) {
+                    const int d0 = (c * 4 + part) * 8;
+                    if (d0 < s.Dp) {
+                        const float4 a = *reinterpret_cast<const float4*>(&sm.q[h][d0]), b = *reinterpret_cast<const float4*>(&sm.q[h][d0 + 4]);
+                        d = fmaf(a.x, kf[c][0], d); d = fmaf(a.y, kf[c][1], d); d = fmaf(a.z, kf[c][2], d); d = fmaf(a.w, kf[c][3], d);
+                        d = fmaf(b.x, kf[c][4], d); d = fmaf(b.y, kf[c][5], d); d = fmaf(b.z, kf[c][6], d); d = fmaf(b.w, kf[c][7], d);
+                    }
+                }
+            }
+            d += __shfl_xor_sync(0xffffffffu, d, 1);
+            d += __shfl_xor_sync(0xffffffffu, d, 2);
+            if (part == 0) {
+                const float slope = s.bias ? distance_slope(h0 + h, s.H) : 0.f;
+                sm.p[h][key] = vis ? d * head_multiplier(s, h0 + h) - slope * (float)(k.pos - k.position(j)) : -INFINITY;
+            }
+        }
+        __syncthreads();
+        // ---- online softmax: one warp per head --------------------------------------------------------------------
+        if (warp < nh && s.shift != nullptr) {                         // weights that need no other key's
+            const float b = __bfloat162float(s.shift[h0 + warp]), s0 = sm.p[warp][lane], s1 = sm.p[warp][lane + 32];
+            sm.p[warp][lane] = s0 == -INFINITY ? 0.f : sigmoid_weight(s0 + b);
+            sm.p[warp][lane + 32] = s1 == -INFINITY ? 0.f : sigmoid_weight(s1 + b);
+            if (lane == 0) sm.alpha[warp] = 1.0f;
+        } else if (warp < nh) {
+            const float s0 = sm.p[warp][lane], s1 = sm.p[warp][lane + 32];
+            const float m_old = sm.m[warp], mn = fmaxf(m_old, warp_max(fmaxf(s0, s1)));       // the tile holds a visible key
+            const float p0 = expf(s0 - mn), p1 = expf(s1 - mn);
+            sm.p[warp][lane] = p0;
+            sm.p[warp][lane + 32] = p1;
+            const float sum = warp_sum(p0 + p1);
+            if (lane == 0) {
+                const float al = expf(m_old - mn);
+                sm.alpha[warp] = al;
+                sm.m[warp] = mn;
+                sm.l[warp] = sm.l[warp] * al + sum;
+            }
+        }
+        __syncthreads();
+        if (pv) {
+#pragma unroll
+            for (int h = 0; h < kHeads; ++h)
+                if (h < nh) {
+                    const float al = sm.alpha[h];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[h][c] *= al;
+                }
+#pragma unroll
+            for (int i = 0; i < VK; ++i) {
+                const int kk = tg + i * kg, jj = j0 + kk;
+                if (kk < kPageTokens && jj < k.end) {
+                    float v[4];
+                    if (jj == k.newest) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) v[c] = sm.vnew[dpart * 4 + c];
+                    } else {
+                        vr[i].get(v);
+                    }
+#pragma unroll
+                    for (int h = 0; h < kHeads; ++h)
+                        if (h < nh) {
+                            const float w = sm.p[h][kk];
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) acc[h][c] = fmaf(w, v[c], acc[h][c]);
+                        }
+                }
+            }
+        }
+        if (j0 + kPageTokens < k.end) load_tile(j0 + kPageTokens);
+        __syncthreads();
+    }
+    // ---- sum over the key groups, then over the splits -------------------------------------------------------------
+    if (pv) {
+#pragma unroll
+        for (int h = 0; h < kHeads; ++h)
+            if (h < nh) *reinterpret_cast<float4*>(sm.red + ((size_t)tg * kHeads + h) * s.Vp + dpart * 4) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+    }
+    __syncthreads();
+    // every output belongs to one block of the cluster: hand it over, then merge the shares locally
+    cl.barrier_wait(std::move(started));
+    const int n_out = nh * s.Dv, share = (n_out + n_splits - 1) / n_splits;
+    for (int i = tid; i < n_out; i += kThreads) {
+        const int h = i / s.Dv, d = i - h * s.Dv;
+        float v = 0.f;
+        for (int t = 0; t < kg; ++t) v += sm.red[((size_t)t * kHeads + h) * s.Vp + d];
+        const int owner = i / share;
+        *cl.map_shared_rank(&sm.rout[split * share + i - owner * share], owner) = v;
+    }
+    for (int i = tid; i < n_splits * kHeads; i += kThreads) {
+        const int r = i / kHeads, h = i - r * kHeads;
+        *cl.map_shared_rank(&sm.rm[split][h], r) = sm.m[h];
+        *cl.map_shared_rank(&sm.rl[split][h], r) = sm.l[h];
+    }
+    cl.sync();
+    for (int i = tid; i < share && split * share + i < n_out; i += kThreads) {
+        const int o = split * share + i, h = o / s.Dv, d = o - h * s.Dv;
+        const float gate = gate_of(h);
+        if (s.shift != nullptr) {
+            float sum = 0.f;
+            for (int r = 0; r < n_splits; ++r) sum += sm.rout[r * share + i];
+            emit(h, d, s.out_scale * gate * sum);
+            continue;
+        }
+        float m = -INFINITY;
+        for (int r = 0; r < n_splits; ++r) m = fmaxf(m, sm.rm[r][h]);
+        float num = 0.f, den = 0.f;
+        for (int r = 0; r < n_splits; ++r) {
+            const float mr = sm.rm[r][h], w = mr == -INFINITY ? 0.f : expf(mr - m);
+            num = fmaf(w, sm.rout[r * share + i], num);
+            den = fmaf(w, sm.rl[r][h], den);
+        }
+        emit(h, d, den > 0.f ? s.out_scale * gate * (num / den) : 0.f);
+    }
+}
+
+// grid (splits = cluster size, kv_heads * head blocks); the visible keys are dealt out evenly, block `split` walks its share in tiles of 64.  VM: upper bound of Dp and Vp.  Further rows of
 // clusters (LIN) compute the linear attention that reads the same projections.
 template <typename TC, int VM, bool ROT, bool LIN>
 __global__ void __launch_bounds__(wd::kThreads) window_attention_decode_kernel(const WindowDecodeParams<TC> p) {
@@ -396,9 +584,6 @@ __global__ void __launch_bounds__(wd::kThreads) window_attention_decode_kernel(c
         }
     }
     const int g = blockIdx.y / hb, h0 = g * group + (blockIdx.y % hb) * kHeads, nh = min(kHeads, (g + 1) * group - h0);
-    const int key = tid >> 2, part = tid & 3;                          // score phase
-    const int tpr = s.Vp / 4, kg = kThreads / tpr, dpart = tid % tpr, tg = tid / tpr;     // P.V phase: 4 channels per thread
-    const bool pv = tg < kg;
 
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -406,34 +591,13 @@ __global__ void __launch_bounds__(wd::kThreads) window_attention_decode_kernel(c
     if (!p.early) { pdl_wait(); pdl_launch_dependents(); }
     const int kv_len = (int)p.state->kv_len, pos = kv_len - 1;
     const bool ok = kv_len > 0 && kv_len <= p.max_pages * kPageTokens;
-    const int lo = s.window > 0 ? max(0, kv_len - s.window) : 0;
-    const int kept = s.window > 0 ? min(s.keep, lo) : 0;               // visible key n stands at position n or, behind the kept ones, n + skip
-    const int skip = lo - kept, n_vis = kv_len - skip, newest = n_vis - 1;
-    const int chunk = ok ? (n_vis + n_splits - 1) / n_splits : 0;
-    const int begin = split * chunk, end = ok ? min(n_vis, begin + chunk) : begin;
+    const SplitKeys k(s, pos, ok, split, n_splits);
 
     Row8<TC> kr[KC];
     Row4<TC> vr[VK];
-    auto position = [&](int n) { return n < kept ? n : n + skip; };
     auto pool_row = [&](int j) { return (size_t)p.pages[j / kPageTokens] * kPageTokens + j % kPageTokens; };
-    // 64 keys from number j0, except the one this launch appends
-    auto load_tile = [&](int j0) {
-        const int j = j0 + key;
-        if (j < end && j != newest) {
-            const TC* src = p.k_pool + (pool_row(position(j)) * s.G + g) * s.Dp;
-#pragma unroll
-            for (int c = 0; c < KC; ++c)
-                if ((c * 4 + part) * 8 < s.Dp) kr[c].load(src + (c * 4 + part) * 8);
-        }
-        if (pv) {
-#pragma unroll
-            for (int i = 0; i < VK; ++i) {
-                const int kk = tg + i * kg, jj = j0 + kk;
-                if (kk < kPageTokens && jj < end && jj != newest) vr[i].load(p.v_pool + (pool_row(position(jj)) * s.G + g) * s.Vp + dpart * 4);
-            }
-        }
-    };
-    if (begin < end) load_tile(begin);
+    auto load_tile = [&](int j0) { window_load_tile(s, k, j0, g, p.k_pool, p.v_pool, pool_row, kr, vr); };
+    if (k.begin < k.end) load_tile(k.begin);
     if constexpr (ROT) {
         if (ok) rot_table(s.rot, pos, sm.cs, sm.sn);
         __syncthreads();
@@ -498,150 +662,56 @@ __global__ void __launch_bounds__(wd::kThreads) window_attention_decode_kernel(c
         sm.vnew[d] = d < s.Dv ? round_as<TC>(__ldcg(p.qkv + (size_t)(s.H + s.G) * s.D + (size_t)g * s.Dv + d)) : 0.f;
     if (tid < kHeads) { sm.m[tid] = -INFINITY; sm.l[tid] = 0.f; }
     __syncthreads();
-    if (begin <= newest && newest < end && blockIdx.y % hb == 0) {     // the block that walks the newest key appends it
+    if (k.begin <= k.newest && k.newest < k.end && blockIdx.y % hb == 0) {     // the block that walks the newest key appends it
         const size_t cr = pool_row(pos);
         for (int d = tid; d < s.Dp; d += kThreads) store_f32(p.k_pool + (cr * s.G + g) * s.Dp + d, sm.knew[d]);
         for (int d = tid; d < s.Vp; d += kThreads) store_f32(p.v_pool + (cr * s.G + g) * s.Vp + d, sm.vnew[d]);
     }
     if (!ok && tid == 0) p.state->error = 2;
 
-    float acc[kHeads][4];
-#pragma unroll
-    for (int h = 0; h < kHeads; ++h)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[h][j] = 0.f;
+    window_split_walk<TC, VM>(sm, s, k, h0, nh, kr, vr, load_tile, cl, started,
+                              [&](int h) { return p.gate != nullptr ? sigmoid_weight(__ldcg(p.gate + h0 + h)) : 1.0f; },
+                              [&](int h, int d, float v) { p.out[(size_t)(h0 + h) * s.Dv + d] = v; });
+}
 
-    for (int j0 = begin; j0 < end; j0 += kPageTokens) {
-        const int j = j0 + key;
-        const bool vis = j < end;
-        // ---- scores: 4 threads per key ----------------------------------------------------------------------------
-        float kf[KC][8];
-#pragma unroll
-        for (int c = 0; c < KC; ++c) {
-            const int d0 = (c * 4 + part) * 8;
-            if (d0 < s.Dp && j == newest) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) kf[c][i] = sm.knew[d0 + i];
-            } else {
-                kr[c].get(kf[c]);
-            }
-        }
-        for (int h = 0; h < nh; ++h) {
-            float d = 0.f;
-            if (vis) {
-#pragma unroll
-                for (int c = 0; c < KC; ++c) {
-                    const int d0 = (c * 4 + part) * 8;
-                    if (d0 < s.Dp) {
-                        const float4 a = *reinterpret_cast<const float4*>(&sm.q[h][d0]), b = *reinterpret_cast<const float4*>(&sm.q[h][d0 + 4]);
-                        d = fmaf(a.x, kf[c][0], d); d = fmaf(a.y, kf[c][1], d); d = fmaf(a.z, kf[c][2], d); d = fmaf(a.w, kf[c][3], d);
-                        d = fmaf(b.x, kf[c][4], d); d = fmaf(b.y, kf[c][5], d); d = fmaf(b.z, kf[c][6], d); d = fmaf(b.w, kf[c][7], d);
-                    }
-                }
-            }
-            d += __shfl_xor_sync(0xffffffffu, d, 1);
-            d += __shfl_xor_sync(0xffffffffu, d, 2);
-            if (part == 0) {
-                const float slope = s.bias ? distance_slope(h0 + h, s.H) : 0.f;
-                sm.p[h][key] = vis ? d * head_multiplier(s, h0 + h) - slope * (float)(pos - position(j)) : -INFINITY;
-            }
-        }
-        __syncthreads();
-        // ---- online softmax: one warp per head --------------------------------------------------------------------
-        if (warp < nh && s.shift != nullptr) {                         // weights that need no other key's
-            const float b = __bfloat162float(s.shift[h0 + warp]), s0 = sm.p[warp][lane], s1 = sm.p[warp][lane + 32];
-            sm.p[warp][lane] = s0 == -INFINITY ? 0.f : sigmoid_weight(s0 + b);
-            sm.p[warp][lane + 32] = s1 == -INFINITY ? 0.f : sigmoid_weight(s1 + b);
-            if (lane == 0) sm.alpha[warp] = 1.0f;
-        } else if (warp < nh) {
-            const float s0 = sm.p[warp][lane], s1 = sm.p[warp][lane + 32];
-            const float m_old = sm.m[warp], mn = fmaxf(m_old, warp_max(fmaxf(s0, s1)));       // the tile holds a visible key
-            const float p0 = expf(s0 - mn), p1 = expf(s1 - mn);
-            sm.p[warp][lane] = p0;
-            sm.p[warp][lane + 32] = p1;
-            const float sum = warp_sum(p0 + p1);
-            if (lane == 0) {
-                const float al = expf(m_old - mn);
-                sm.alpha[warp] = al;
-                sm.m[warp] = mn;
-                sm.l[warp] = sm.l[warp] * al + sum;
-            }
-        }
-        __syncthreads();
-        if (pv) {
-#pragma unroll
-            for (int h = 0; h < kHeads; ++h)
-                if (h < nh) {
-                    const float al = sm.alpha[h];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[h][c] *= al;
-                }
-#pragma unroll
-            for (int i = 0; i < VK; ++i) {
-                const int kk = tg + i * kg, jj = j0 + kk;
-                if (kk < kPageTokens && jj < end) {
-                    float v[4];
-                    if (jj == newest) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) v[c] = sm.vnew[dpart * 4 + c];
-                    } else {
-                        vr[i].get(v);
-                    }
-#pragma unroll
-                    for (int h = 0; h < kHeads; ++h)
-                        if (h < nh) {
-                            const float w = sm.p[h][kk];
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) acc[h][c] = fmaf(w, v[c], acc[h][c]);
-                        }
-                }
-            }
-        }
-        if (j0 + kPageTokens < end) load_tile(j0 + kPageTokens);
-        __syncthreads();
+// ---- rows of short entries -----------------------------------------------------------------------------------------
+// One cluster per row and kv head, on queries that are normed and rotated already and a cache that holds the row's own key: decoded
+// tokens of many sequences, short portions.  A block of window_attention_rows serves 16 rows of an entry with one head and reads the
+// keys one tile of 32 after the other: with one row in it that is all serial latency on an idle chip.  Here the keys of a row are split
+// over the blocks of a cluster, a block serves all heads of a kv head and requests a tile ahead.  Bound: latency (16 rows that see
+// 1040 keys, 16 heads on 4 kv heads of 128 channels: 17 MB).  16 such rows beside a portion of 200: 679 us a layer with 16-row blocks,
+// a step of 8 layers 6.1 ms; 3.5 ms with this kernel.
+template <typename T, int VM>
+__global__ void __launch_bounds__(wd::kThreads) window_attention_short_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool,
+                                                                              T* __restrict__ out, int ld_out, const WindowAttnShape s, const RowPlan plan,
+                                                                              const int32_t* __restrict__ rows) {
+    using namespace wd;
+    constexpr int KC = VM / 32, VK = VM <= 64 ? 4 : (VM <= 128 ? 8 : 16);
+    extern __shared__ __align__(16) unsigned char wd_smem[];
+    Smem<VM>& sm = *reinterpret_cast<Smem<VM>*>(wd_smem);
+    const int tid = threadIdx.x, row = rows != nullptr ? rows[blockIdx.z] : (int)blockIdx.z;
+    const int group = s.H / s.G, hb = (group + kHeads - 1) / kHeads;
+    const int g = blockIdx.y / hb, h0 = g * group + (blockIdx.y % hb) * kHeads, nh = min(kHeads, (g + 1) * group - h0);
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    auto started = cl.barrier_arrive();
+    const RowEntry e = plan.of_row(row);
+    SplitKeys k(s, e.pos0 + row - e.row0, true, blockIdx.x, gridDim.x);
+    k.newest = -1;
+    Row8<T> kr[KC];
+    Row4<T> vr[VK];
+    auto pool_row = [&](int j) { return plan.cache_row(e, j); };
+    auto load_tile = [&](int j0) { window_load_tile(s, k, j0, g, k_pool, v_pool, pool_row, kr, vr); };
+    if (k.begin < k.end) load_tile(k.begin);
+    for (int i = tid; i < nh * s.Dp; i += kThreads) {
+        const int h = i / s.Dp, d = i - h * s.Dp;
+        sm.q[h][d] = to_f32(q[((size_t)row * s.H + h0 + h) * s.Dp + d]);
     }
-    // ---- sum over the key groups, then over the splits -------------------------------------------------------------
-    if (pv) {
-#pragma unroll
-        for (int h = 0; h < kHeads; ++h)
-            if (h < nh) *reinterpret_cast<float4*>(sm.red + ((size_t)tg * kHeads + h) * s.Vp + dpart * 4) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
-    }
+    if (tid < kHeads) { sm.m[tid] = -INFINITY; sm.l[tid] = 0.f; }
     __syncthreads();
-    // every output belongs to one block of the cluster: hand it over, then merge the shares locally
-    cl.barrier_wait(std::move(started));
-    const int n_out = nh * s.Dv, share = (n_out + n_splits - 1) / n_splits;
-    for (int i = tid; i < n_out; i += kThreads) {
-        const int h = i / s.Dv, d = i - h * s.Dv;
-        float v = 0.f;
-        for (int t = 0; t < kg; ++t) v += sm.red[((size_t)t * kHeads + h) * s.Vp + d];
-        const int owner = i / share;
-        *cl.map_shared_rank(&sm.rout[split * share + i - owner * share], owner) = v;
-    }
-    for (int i = tid; i < n_splits * kHeads; i += kThreads) {
-        const int r = i / kHeads, h = i - r * kHeads;
-        *cl.map_shared_rank(&sm.rm[split][h], r) = sm.m[h];
-        *cl.map_shared_rank(&sm.rl[split][h], r) = sm.l[h];
-    }
-    cl.sync();
-    for (int i = tid; i < share && split * share + i < n_out; i += kThreads) {
-        const int o = split * share + i, h = o / s.Dv, d = o - h * s.Dv;
-        const float gate = p.gate != nullptr ? sigmoid_weight(__ldcg(p.gate + h0 + h)) : 1.0f;
-        if (s.shift != nullptr) {
-            float sum = 0.f;
-            for (int r = 0; r < n_splits; ++r) sum += sm.rout[r * share + i];
-            p.out[(size_t)(h0 + h) * s.Dv + d] = s.out_scale * gate * sum;
-            continue;
-        }
-        float m = -INFINITY;
-        for (int r = 0; r < n_splits; ++r) m = fmaxf(m, sm.rm[r][h]);
-        float num = 0.f, den = 0.f;
-        for (int r = 0; r < n_splits; ++r) {
-            const float mr = sm.rm[r][h], w = mr == -INFINITY ? 0.f : expf(mr - m);
-            num = fmaf(w, sm.rout[r * share + i], num);
-            den = fmaf(w, sm.rl[r][h], den);
-        }
-        p.out[(size_t)(h0 + h) * s.Dv + d] = den > 0.f ? s.out_scale * gate * (num / den) : 0.f;
-    }
+    window_split_walk<T, VM>(sm, s, k, h0, nh, kr, vr, load_tile, cl, started,
+                             [&](int h) { return s.gate != nullptr ? sigmoid_weight(to_f32(static_cast<const T*>(s.gate)[(size_t)row * s.gate_ld + h0 + h])) : 1.0f; },
+                             [&](int h, int d, float v) { store_f32(out + (size_t)row * ld_out + (size_t)(h0 + h) * s.Dv + d, v); });
 }
 
 }  // namespace efm

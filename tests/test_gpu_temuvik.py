@@ -157,6 +157,25 @@ def test_a_batch_is_each_request_alone(mixed):
         assert tu.error(np.concatenate(rows[k]), alone[k]) < (1e-5 if limit < 1e-3 else 2e-2)
 
 
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("live,window", [(2, None), (14, 65), (14, None), (40, 130), (150, None)])
+def test_short_entries_of_a_full_batch(built, tmp_path, live, window, dtype):
+    """One to three rows of many requests in one step: the keys of a row are split over 16 blocks (2 live ones) down to one (150)."""
+    cfg = config([attention(heads=8, kv_heads=2, dim=64, vdim=40, size=window, keep=5, rot=64), attention(heads=9, kv_heads=1, dim=24, vdim=72, size=window, keep=70, rot=16)],
+                 width=64, vocab=60)
+    w = tu.weights(cfg, seed=9)
+    lengths = [(1 + 37 * i) % 210 + 1 for i in range(live)]
+    lengths[0] = 1100 if window is None and live < 100 else 64
+    seq = tu.tokens(cfg, max(lengths) + 3)
+    ref = reference(cfg, w, seq).logits.numpy()
+    eng = tu.engine(tmp_path, cfg, w, dtype, pool=64 * sum((n + 66) // 64 for n in lengths), live=live)
+    for i, n in enumerate(lengths):
+        tu.step(eng, [("r%d" % i, seq[:n], [])])
+    entries = [("r%d" % i, seq[n:n + 1 + i % 3], list(range(1 + i % 3))) for i, n in enumerate(lengths)]
+    got = tu.step(eng, entries)
+    assert tu.error(got, np.concatenate([ref[n:n + 1 + i % 3] for i, n in enumerate(lengths)])) < tu.LIMIT[dtype]
+
+
 def test_steps_longer_than_one_pass(built, tmp_path):
     cfg = config([attention(size=50), latent(size=40, mlp=experts())], vocab=64, loop=(0, 2, 2))
     w = tu.weights(cfg, seed=2)
