@@ -41,6 +41,7 @@ Launcher make_launcher(efm_b200_ctx* c) {
     Launcher L;
     L.stream = c->stream;
     L.pdl = c->pdl;
+    L.rows = c->pdl && c->tp_size <= 1;
     L.counter = &c->launches;
     L.gemm_ws = c->gemm_ws;
     L.gemm_ws_floats = c->gemm_ws_floats;
@@ -234,6 +235,7 @@ efm_status efm_b200_prefill(efm_b200_ctx* c, int32_t slot, const int32_t* token_
         if (!tail) return;
         const bool w4 = c->decode_w4;
         c->decode_w4 = false;            // the first token belongs to the prefill pass: bf16 weights even when decode runs on INT4
+        LL.joined = true;                // the step may read the cache ahead of its waits: not before the rows' pass is over
         c->ops->decode_step(*c, s, LL);
         c->decode_w4 = w4;
     };

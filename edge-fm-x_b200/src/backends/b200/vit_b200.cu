@@ -397,6 +397,7 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
     Launcher L;
     L.stream = st;
     L.pdl = false;
+    L.rows = c->pdl;
     L.counter = &c->launches;
     L.gemm_ws = c->gemm_ws;
     L.gemm_ws_floats = c->gemm_ws_floats;
@@ -416,11 +417,11 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
         GemmParams g{px, v->patch_w, nullptr, nullptr, v->pe, N, H, v->patch_dim};
         launch_gemm_epi(L, GemmEpi::F32, g, err);
         if (nm > 0)
-            L.launch(vit_gather_blocks_f32_kernel, dim3(std::min(nm, c->num_sms * 8)), dim3(256), 0, (const float*)v->pe, v->resid,
+            L.launch_rows(vit_gather_blocks_f32_kernel, dim3(std::min(nm, c->num_sms * 8)), dim3(256), 0, (const float*)v->pe, v->resid,
                      (const int32_t*)(order + r0 / v->unit), nm, v->unit, H);
     }
     if (n > 0)
-        L.launch(vit_rope_table_kernel, dim3((n * (D / 2) + 127) / 128), dim3(128), 0, v->rope_tab, (const int32_t*)(pos_h + r0),
+        L.launch_rows(vit_rope_table_kernel, dim3((n * (D / 2) + 127) / 128), dim3(128), 0, v->rope_tab, (const int32_t*)(pos_h + r0),
                  (const int32_t*)(pos_w + r0), n, D, d.rope_theta);
     for (int l = 0; l < d.depth; ++l) {
         const VitBlock& b = v->blocks[l];
@@ -430,7 +431,7 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
         if (n > 0) {
             GemmParams g{v->xn, b.qkv_w, b.qkv_b, v->qkv, nullptr, n, 3 * H, H};
             launch_gemm_epi(L, GemmEpi::Bf16Bias, g, err);
-            L.launch(vit_rope2d_kernel, dim3(n), dim3(256), 0, v->qkv, (const float2*)v->rope_tab, d.heads, D);
+            L.launch_rows(vit_rope2d_kernel, dim3(n), dim3(256), 0, v->qkv, (const float2*)v->rope_tab, d.heads, D);
         }
         const __nv_bfloat16* kv_rows = v->qkv;
         if (full && tp > 1) {
@@ -474,7 +475,7 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
             merged = v->mo_all;
         }
         __nv_bfloat16* dst = out_mem == EFM_MEM_DEVICE ? static_cast<__nv_bfloat16*>(out) : v->out_dev;
-        L.launch(vit_scatter_rows_bf16_kernel, dim3(std::min(NM, c->num_sms * 8)), dim3(128), 0, merged, dst,
+        L.launch_rows(vit_scatter_rows_bf16_kernel, dim3(std::min(NM, c->num_sms * 8)), dim3(128), 0, merged, dst,
                  (const int32_t*)order, NM, d.out_hidden);
     }
     if (L.err != cudaSuccess) return vfail(v, EFM_ERR_CUDA, std::string("vision encoder launch: ") + cudaGetErrorString(L.err));

@@ -420,6 +420,7 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
 
     auto mark = [&](int i) { if (v->mark_phases && L.err == cudaSuccess) L.err = cudaEventRecord(v->phase_ev[i], L.stream); };
     mark(0);
+    L.rows = true;
     // the action state starts as the noise (copied here, far ahead of the loop that launches with programmatic edges)
     if (L.err == cudaSuccess) L.err = cudaMemcpyAsync(v->x_t, v->noise, (size_t)n * d.action_dim * 4, cudaMemcpyDeviceToDevice, L.stream);
     auto layernorm = [&](const __nv_bfloat16* w, const __nv_bfloat16* b) {       // v_resid -> v_xn
@@ -503,7 +504,7 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
     // the loop's kernels all open with the dependent-launch wait, so they may be launched with programmatic
     // serialization (off by default, see use_pdl; the tcgen05 GEMM of the chunk > 64 fallback has no such wait)
     L.pdl = skinny && v->use_pdl;
-    L.pdl_rows = L.pdl;
+    L.rows = L.pdl;
     for (int s = 0; s < d.steps; ++s) {
         if (skinny) {      // the two wider linears of the suffix embedding on the weight-streaming kernel, bf16 activations
             small(0, v->x_t, d.action_dim, v->ain_w, v->ain_b, v->cat, 2 * He, n, He, d.action_dim, 0.f, v->cat16, 2 * He);
@@ -558,7 +559,7 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
         small(0, v->hf, He, v->aout_w, v->aout_b, v->x_t, d.action_dim, n, d.action_dim, He, dt);
     }
     L.pdl = false;
-    L.pdl_rows = false;
+    L.rows = false;
     mark(4);
 }
 

@@ -15,10 +15,7 @@ static void launch_seg_attention_dn(Launcher& L, const SegAttnParams& p) {
         attr_set = true;
     }
     const dim3 grid((p.S + 16 * NW - 1) / (16 * NW), p.q_heads), block(32 * NW);
-    const bool pdl = L.pdl;
-    L.pdl = pdl && L.pdl_rows;
-    L.launch(seg_attention_kernel<D, NW>, grid, block, sa::smem_bytes<D, NW>(), p);
-    L.pdl = pdl;
+    L.launch_rows(seg_attention_kernel<D, NW>, grid, block, sa::smem_bytes<D, NW>(), p);
 }
 
 template <int D>
@@ -39,10 +36,7 @@ void launch_seg_attention_short(Launcher& L, const SegAttnParams& p, int D, int 
         cudaFuncSetAttribute(seg_attention_kernel<64, 4, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sa::smem_bytes<64, 4, PRE>());
         attr_set = true;
     }
-    const bool pdl = L.pdl;
-    L.pdl = pdl && L.pdl_rows;
-    L.launch(seg_attention_kernel<64, 4, PRE>, dim3(1, p.q_heads), dim3(128), sa::smem_bytes<64, 4, PRE>(), p);
-    L.pdl = pdl;
+    L.launch_rows(seg_attention_kernel<64, 4, PRE>, dim3(1, p.q_heads), dim3(128), sa::smem_bytes<64, 4, PRE>(), p);
 }
 
 bool attention_tc_enabled() {
@@ -65,10 +59,7 @@ static bool launch_seg_attention_tc_d(Launcher& L, const SegAttnParams& p0) {
     const uint64_t kd[3] = {(uint64_t)D, (uint64_t)p.kv_heads, (uint64_t)p.kv_rows}, ks[2] = {(uint64_t)D * 2, (uint64_t)p.kv_stride * 2};
     const uint32_t qb[3] = {64, 1, (uint32_t)at::BM}, kb[3] = {64, 1, (uint32_t)at::BN};
     if (!make_map_nd(&mq, p.q, 3, qd, qs, qb) || !make_map_nd(&mk, p.k, 3, kd, ks, kb) || !make_map_nd(&mv, p.v, 3, kd, ks, kb)) return false;
-    const bool pdl = L.pdl;
-    L.pdl = false;
-    L.launch(seg_attention_tc_kernel<D>, dim3((p.S + at::BM - 1) / at::BM, p.q_heads), dim3(at::kThreads), C::SMEM, mq, mk, mv, p, p.error);
-    L.pdl = pdl;
+    L.launch_rows(seg_attention_tc_kernel<D>, dim3((p.S + at::BM - 1) / at::BM, p.q_heads), dim3(at::kThreads), C::SMEM, mq, mk, mv, p, p.error);
     return true;
 }
 

@@ -235,7 +235,7 @@ void launch_attn_short_v(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, co
     while (splits < pages && splits < m.attn_cluster && (int64_t)2 * splits * s.G * hb * n <= 4 * c.num_sms) splits *= 2;
     for (int r0 = 0; r0 < n; r0 += 32768) {                          // grid.z
         L.cluster_x = splits;
-        L.launch(window_attention_short_kernel<T, VM>, dim3(splits, s.G * hb, std::min(n - r0, 32768)), dim3(wd::kThreads), sizeof(wd::Smem<VM>),
+        L.launch_rows(window_attention_short_kernel<T, VM>, dim3(splits, s.G * hb, std::min(n - r0, 32768)), dim3(wd::kThreads), sizeof(wd::Smem<VM>),
                  static_cast<const T*>(m.q), static_cast<const T*>(run.k_pool), static_cast<const T*>(run.v_pool), static_cast<T*>(m.mix), l.mix_wp, s, plan,
                  rows != nullptr ? rows + r0 : nullptr);
     }
@@ -575,7 +575,7 @@ namespace {
 // out[rows, w.Np] = a[rows, w.Kp] . w^T.  bf16 activations run on the tensor cores, fp32 ones in fp32 FMAs.
 void linear_f32(efm_b200_ctx& c, Launcher& L, const DecLinear& w, const void* a, float* out, int rows) {
     if (c.decoder->f32) {
-        L.launch(gemm_f32_kernel, dim3((w.Np + 63) / 64, (rows + 63) / 64), dim3(256), 0, static_cast<const float*>(a), w.Kp,
+        L.launch_rows(gemm_f32_kernel, dim3((w.Np + 63) / 64, (rows + 63) / 64), dim3(256), 0, static_cast<const float*>(a), w.Kp,
                  (const __nv_bfloat16*)w.w, w.Kp, out, w.Np, rows, w.Np, w.Kp, (const __nv_bfloat16*)w.bias, RowGroups{});
         return;
     }
@@ -645,7 +645,7 @@ void launch_latent_tc(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const
     const LatentShape z = latent_shape(m, l);
     const int LR = z.Lc + z.Rc, n_ws = tiles.n_ws * kPageTokens, ld = l.ukv.Np;
     if (tiles.n_gather > 0)
-        L.launch(latent_gather_rows_kernel<__nv_bfloat16>, dim3(tiles.n_gather, 4), dim3(256), 0, static_cast<const __nv_bfloat16*>(run.k_pool), m.ws_c, LR, plan,
+        L.launch_rows(latent_gather_rows_kernel<__nv_bfloat16>, dim3(tiles.n_gather, 4), dim3(256), 0, static_cast<const __nv_bfloat16*>(run.k_pool), m.ws_c, LR, plan,
                  tiles.ws_pages, tiles.ws_page0);
     GemmParams g{m.ws_c, l.ukv.w, nullptr, m.ws_kv, nullptr, n_ws, l.ukv.Np, l.ukv.Kp};
     g.lda = LR;
@@ -672,9 +672,9 @@ void launch_delta_chunks(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, co
     DecoderModel& m = *c.decoder;
     const DeltaShape s = delta_shape(m, l);
     const int chunks = plan.n_entries == 1 ? (plan.rows + dc::C - 1) / dc::C : plan.rows / dc::C + plan.n_entries;     // at most
-    L.launch(delta_prepare_kernel<DP>, dim3(chunks, l.d.heads), dim3(dc::kThreads), sizeof(dc::PrepSmem<DP>), (const float*)m.proj_f, (const float*)m.decay,
+    L.launch_rows(delta_prepare_kernel<DP>, dim3(chunks, l.d.heads), dim3(dc::kThreads), sizeof(dc::PrepSmem<DP>), (const float*)m.proj_f, (const float*)m.decay,
              l.w2.Np, m.pack, s, plan);
-    L.launch(delta_chunk_scan_kernel<DP>, dim3(l.d.heads * (DP / dc::kCols), plan.n_entries), dim3(dc::kScanThreads), sizeof(dc::ScanSmem<DP>), (const float*)m.pack,
+    L.launch_rows(delta_chunk_scan_kernel<DP>, dim3(l.d.heads * (DP / dc::kCols), plan.n_entries), dim3(dc::kScanThreads), sizeof(dc::ScanSmem<DP>), (const float*)m.pack,
              m.o, l.mix_wp, m.state_pool, m.state_stride, run.state_off, s, plan);
 }
 
@@ -712,7 +712,7 @@ void linear_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const Deco
         else decay_product(std::integral_constant<int, 32>{});
     } else if (s.rank > 0) {                                           // W_a2 W_a1 x + b, then the decays it stands for
         if (m.f32) {
-            L.launch(gemm_f32_kernel, dim3((l.w2.Np + 63) / 64, (plan.rows + 63) / 64), dim3(256), 0, reinterpret_cast<const float*>(proj) + s.off_a, s.ld,
+            L.launch_rows(gemm_f32_kernel, dim3((l.w2.Np + 63) / 64, (plan.rows + 63) / 64), dim3(256), 0, reinterpret_cast<const float*>(proj) + s.off_a, s.ld,
                      (const __nv_bfloat16*)l.w2.w, l.w2.Kp, m.decay, l.w2.Np, plan.rows, l.w2.Np, l.w2.Kp, (const __nv_bfloat16*)l.w2.bias, RowGroups{});
         } else {
             GemmParams g{reinterpret_cast<const __nv_bfloat16*>(proj) + s.off_a, l.w2.w, l.w2.bias, nullptr, m.decay, plan.rows, l.w2.Np, l.w2.Kp};
@@ -831,11 +831,11 @@ void attention_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const D
     TA* vp = static_cast<TA*>(run.v_pool);
     int lanes = 8;                                                  // 8 channels each: at most 256 (padded) channels a head
     while (lanes * 8 < std::max(s.Dp, s.Vp)) lanes *= 2;
-    L.launch(s.rot.kind != kRotNone ? qk_scatter_rows_kernel<TA, TA, TA, true> : qk_scatter_rows_kernel<TA, TA, TA, false>, dim3(plan.rows), dim3(256), 0,
+    L.launch_rows(s.rot.kind != kRotNone ? qk_scatter_rows_kernel<TA, TA, TA, true> : qk_scatter_rows_kernel<TA, TA, TA, false>, dim3(plan.rows), dim3(256), 0,
              static_cast<const TA*>(m.proj_a), l.in.Np, static_cast<TA*>(m.q), kp, vp, s, plan, lanes);
     auto cuda_cores = [&](const RowTile* list, int n) {
         if (n > 0)
-            L.launch(window_attention_rows_kernel<TA, TA, TA>, dim3(n, s.H), dim3(256), wa::rows_smem_bytes(s.Dp, s.Vp), static_cast<const TA*>(m.q),
+            L.launch_rows(window_attention_rows_kernel<TA, TA, TA>, dim3(n, s.H), dim3(256), wa::rows_smem_bytes(s.Dp, s.Vp), static_cast<const TA*>(m.q),
                      (const TA*)kp, (const TA*)vp, static_cast<TA*>(m.mix), l.mix_wp, s, plan, list);
     };
     if (tiles.listed && tiles.n_short > 0) launch_attn_short<TA>(c, L, l, run, s, plan, tiles.short_rows, tiles.n_short);
@@ -863,10 +863,10 @@ void latent_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const Deco
     if constexpr (std::is_same<TA, __nv_bfloat16>::value) {
         if (decoder_layer_tc(m, l)) ws = m.ws_c;
     }
-    L.launch(latent_rows_kernel<TA>, dim3((T + kLatentRowsPerBlock - 1) / kLatentRowsPerBlock), dim3(32 * kLatentRowsPerBlock), 0, static_cast<const TA*>(m.proj_a),
+    L.launch_rows(latent_rows_kernel<TA>, dim3((T + kLatentRowsPerBlock - 1) / kLatentRowsPerBlock), dim3(32 * kLatentRowsPerBlock), 0, static_cast<const TA*>(m.proj_a),
              l.in.Np, static_cast<TA*>(m.cq), static_cast<TA*>(run.k_pool), ws, kTcMinRows, s, plan);
     linear_act(c, L, l.uq, m.cq, m.q, T);
-    L.launch(latent_rotate_rows_kernel<TA>, dim3(T), dim3(256), 0, static_cast<TA*>(m.q), s, plan);
+    L.launch_rows(latent_rotate_rows_kernel<TA>, dim3(T), dim3(256), 0, static_cast<TA*>(m.q), s, plan);
     if constexpr (std::is_same<TA, __nv_bfloat16>::value) {
         if (decoder_layer_tc(m, l)) {
             if (tiles.listed) {
@@ -896,6 +896,7 @@ SumOf<TA> expert_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const
     Launcher S = L;
     S.stream = m.side;
     S.gemm_ws = nullptr;
+    S.rows = false;
     auto order = [&](cudaError_t e) { if (L.err == cudaSuccess) L.err = e; };
     if (l.d.shared_ff > 0) order(cudaEventRecord(m.side_start, L.stream));
     linear_f32(c, L, l.router, h, m.route_logits, T);
@@ -915,14 +916,14 @@ SumOf<TA> expert_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const
         order(S.err);
         order(cudaEventRecord(m.side_end, m.side));
     }
-    L.launch(expert_route_rows_kernel, dim3((T + 7) / 8), dim3(256), 0, (const float*)m.route_logits, l.router.Np, T, r, m.ex);
-    L.launch(l.d.expert_weight_input ? expert_gather_rows_kernel<TA, true> : expert_gather_rows_kernel<TA, false>, dim3(T), dim3(128), 0, static_cast<const TA*>(h), static_cast<TA*>(m.ex_in), m.Wp, r, m.ex);
+    L.launch_rows(expert_route_rows_kernel, dim3((T + 7) / 8), dim3(256), 0, (const float*)m.route_logits, l.router.Np, T, r, m.ex);
+    L.launch_rows(l.d.expert_weight_input ? expert_gather_rows_kernel<TA, true> : expert_gather_rows_kernel<TA, false>, dim3(T), dim3(128), 0, static_cast<const TA*>(h), static_cast<TA*>(m.ex_in), m.Wp, r, m.ex);
     // tiles in use at most: every row tile but the last of an expert is full
     const int64_t picks = (int64_t)T * r.top;
     const int max_rows = (int)std::min<int64_t>(m.ex_rows, (picks / kExpertTile + std::min<int64_t>(picks, r.experts)) * kExpertTile);
     if constexpr (std::is_same<TA, float>::value) {
         auto product = [&](const DecLinear& w, int n, const float* a, float* out) {
-            L.launch(gemm_f32_kernel, dim3((n + 63) / 64, (max_rows + 63) / 64), dim3(256), 0, a, w.Kp, (const __nv_bfloat16*)w.w, w.Kp, out, n, max_rows, n, w.Kp,
+            L.launch_rows(gemm_f32_kernel, dim3((n + 63) / 64, (max_rows + 63) / 64), dim3(256), 0, a, w.Kp, (const __nv_bfloat16*)w.w, w.Kp, out, n, max_rows, n, w.Kp,
                      (const __nv_bfloat16*)nullptr, RowGroups{m.ex.tile, m.ex.n_tiles, n});
         };
         product(l.expert_in, l.up_rows(l.ffp), static_cast<const float*>(m.ex_in), m.ex_gu);
@@ -942,7 +943,10 @@ SumOf<TA> expert_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const
         product(l.expert_in, l.up_rows(l.ffp), expert_epi(l), m.ex_in, m.ex_act);
         product(l.expert_out, m.Wp, GemmEpi::Bf16Bias, m.ex_act, m.ex_y);
     }
-    if (l.d.shared_ff > 0) order(cudaStreamWaitEvent(L.stream, m.side_end, 0));
+    if (l.d.shared_ff > 0) {
+        order(cudaStreamWaitEvent(L.stream, m.side_end, 0));
+        L.joined = true;
+    }
     return SumOf<TA>{static_cast<const TA*>(m.ex_y), m.ex.place, m.ex.weight, r.top, m.ex.count, r.experts, l.d.expert_weight_input,
                      l.d.shared_ff > 0 ? static_cast<const TA*>(m.sh_y) : nullptr, m.ex.shared};
 }
@@ -952,8 +956,8 @@ void delta_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const Decod
     DecoderModel& m = *c.decoder;
     const DeltaShape s = delta_shape(m, l);
     linear_f32(c, L, l.in, x, m.proj_f, plan.rows);
-    L.launch(delta_tanh_rows_kernel, dim3(plan.rows), dim3(128), 0, (const float*)m.proj_f, m.tanh_w, l.w2.Kp, s);
-    L.launch(gemm_f32_kernel, dim3((l.w2.Np + 63) / 64, (plan.rows + 63) / 64), dim3(256), 0, (const float*)m.tanh_w, l.w2.Kp, (const __nv_bfloat16*)l.w2.w,
+    L.launch_rows(delta_tanh_rows_kernel, dim3(plan.rows), dim3(128), 0, (const float*)m.proj_f, m.tanh_w, l.w2.Kp, s);
+    L.launch_rows(gemm_f32_kernel, dim3((l.w2.Np + 63) / 64, (plan.rows + 63) / 64), dim3(256), 0, (const float*)m.tanh_w, l.w2.Kp, (const __nv_bfloat16*)l.w2.w,
              l.w2.Kp, m.decay, l.w2.Np, plan.rows, l.w2.Np, l.w2.Kp, (const __nv_bfloat16*)nullptr, RowGroups{});
     const bool chunked = plan.rows >= dc::C && s.Dp <= 128;         // short passes and larger heads: token by token
     if (chunked) {
@@ -978,7 +982,7 @@ void delta_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const Decod
     }
     int lanes = 1;
     while (lanes * 4 < s.D && lanes < 32) lanes *= 2;
-    L.launch(delta_output_rows_kernel<TA>, dim3(plan.rows), dim3(256), 0, (const float*)m.o, l.mix_wp, (const float*)m.proj_f, static_cast<TA*>(m.mix), l.mix_wp,
+    L.launch_rows(delta_output_rows_kernel<TA>, dim3(plan.rows), dim3(256), 0, (const float*)m.o, l.mix_wp, (const float*)m.proj_f, static_cast<TA*>(m.mix), l.mix_wp,
              s, lanes);
 }
 
@@ -1001,12 +1005,12 @@ void rows_pass(efm_b200_ctx& c, const RowPlan& plan, const int32_t* ids, const R
             return;
         }
         if (avg != nullptr) {
-            L.launch(experts ? add_norm_rows_kernel<TA, false, true, true> : add_norm_rows_kernel<TA, false, false, true>, dim3(T), dim3(256), 0, c.resid, stream, y, w,
+            L.launch_rows(experts ? add_norm_rows_kernel<TA, false, true, true> : add_norm_rows_kernel<TA, false, false, true>, dim3(T), dim3(256), 0, c.resid, stream, y, w,
                      (TA*)nullptr, (const __nv_bfloat16*)nullptr, m.W, m.Wp, m.d.norm_eps, sum, *avg);
             stream = c.resid;
             return;
         }
-        L.launch(pre != nullptr ? (experts ? add_norm_rows_kernel<TA, true, true> : add_norm_rows_kernel<TA, true, false>)
+        L.launch_rows(pre != nullptr ? (experts ? add_norm_rows_kernel<TA, true, true> : add_norm_rows_kernel<TA, true, false>)
                                 : (experts ? add_norm_rows_kernel<TA, false, true> : add_norm_rows_kernel<TA, false, false>),
                  dim3(T), dim3(256), 0, c.resid, stream, y, w, m.d.conv_taps > 0 ? (TA*)nullptr : xa, pre, m.W, m.Wp, m.d.norm_eps, sum, DepthAverage{});
         stream = c.resid;
@@ -1060,7 +1064,7 @@ void rows_pass(efm_b200_ctx& c, const RowPlan& plan, const int32_t* ids, const R
             const bool poly = l.d.ff_act == EFM_ACT_POLYNORM;
             if (poly) {
                 linear_act(c, L, l.up, xin, m.ff, T);
-                L.launch(poly_norm_rows_kernel<TA>, dim3(T), dim3(256), 0, static_cast<const TA*>(m.ff), static_cast<TA*>(m.ff2), (const __nv_bfloat16*)l.act, l.d.ff,
+                L.launch_rows(poly_norm_rows_kernel<TA>, dim3(T), dim3(256), 0, static_cast<const TA*>(m.ff), static_cast<TA*>(m.ff2), (const __nv_bfloat16*)l.act, l.d.ff,
                          l.down.Kp, m.d.norm_eps);
             } else if (m.f32) {
                 linear_f32(c, L, l.up, xin, static_cast<float*>(m.ff), T);
@@ -1074,7 +1078,7 @@ void rows_pass(efm_b200_ctx& c, const RowPlan& plan, const int32_t* ids, const R
         }
         if (m.d.side_dim > 0) {
             linear_f32(c, L, l.gate, xin, m.side_f, T);
-            L.launch(token_gate_rows_kernel<TA>, dim3(T), dim3(128), 0, (const float*)m.side_f, ids, (const __nv_bfloat16*)m.side_embed,
+            L.launch_rows(token_gate_rows_kernel<TA>, dim3(T), dim3(128), 0, (const float*)m.side_f, ids, (const __nv_bfloat16*)m.side_embed,
                      m.d.side_dim * m.d.num_layers, run.layer * m.d.side_dim, c.d.vocab, static_cast<TA*>(m.side_a), m.d.side_dim, m.side_p);
             linear_f32(c, L, l.proj, m.side_a, m.y, T);
             add_norm(m.y, l.side_norm, DecNorm{});
@@ -1105,7 +1109,7 @@ void decoder_rows_logits(efm_b200_ctx& c, const int32_t* rows, int n, Launcher& 
             L.launch(gather_tanh_rows_kernel<TA>, dim3(n), dim3(256), 0, (const float*)c.resid, rows, (const __nv_bfloat16*)f.w, (const __nv_bfloat16*)f.b,
                      (const __nv_bfloat16*)f.alpha, out, m.Wp);
         else
-            L.launch(gather_norm_rows_kernel<TA>, dim3(n), dim3(256), 0, (const float*)c.resid, rows, (const __nv_bfloat16*)f.w, out, m.W, m.Wp, m.d.norm_eps);
+            L.launch_rows(gather_norm_rows_kernel<TA>, dim3(n), dim3(256), 0, (const float*)c.resid, rows, (const __nv_bfloat16*)f.w, out, m.W, m.Wp, m.d.norm_eps);
     };
     if (m.f32) gather(static_cast<float*>(m.head_a));
     else gather(static_cast<__nv_bfloat16*>(m.head_a));

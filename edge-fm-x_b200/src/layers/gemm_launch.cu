@@ -75,8 +75,6 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
     }
     const int tiles = ((p.N + tc::BN - 1) / tc::BN) * ((p.M + tc::BM - 1) / tc::BM);
     const dim3 block(tc::kThreads);
-    const bool pdl = L.pdl;
-    L.pdl = false;     // prefill kernels do not use the dependent-launch protocol
     if constexpr (EPI == GemmEpi::Bf16Bias || EPI == GemmEpi::Bf16Relu2 || gemm_is_glu(EPI)) {
         if (p.group_tile != nullptr) {
             static bool attr_group = false;
@@ -84,8 +82,7 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
                 cudaFuncSetAttribute(gemm_tc_kernel<EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM_BYTES);
                 attr_group = true;
             }
-            L.launch(gemm_tc_kernel<EPI, true>, dim3(std::min(L.num_sms, tiles)), block, tc::SMEM_BYTES, ma, mb, p, error_word);
-            L.pdl = pdl;
+            L.launch_rows(gemm_tc_kernel<EPI, true>, dim3(std::min(L.num_sms, tiles)), block, tc::SMEM_BYTES, ma, mb, p, error_word);
             return;
         }
     }
@@ -108,11 +105,10 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
                 cudaFuncSetAttribute(gemm_tc_kernel<GemmEpi::F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM_BYTES);
                 attr_f32 = true;
             }
-            L.launch(gemm_tc_kernel<GemmEpi::F32>, dim3(std::min(L.num_sms, tiles * splits)), block, tc::SMEM_BYTES, ma, mb, q, error_word);
+            L.launch_rows(gemm_tc_kernel<GemmEpi::F32>, dim3(std::min(L.num_sms, tiles * splits)), block, tc::SMEM_BYTES, ma, mb, q, error_word);
             const size_t total4 = (size_t)p.M * p.N / (gemm_is_glu(EPI) ? 8 : 4);
             const int fin = (int)std::min<size_t>((total4 + 255) / 256, (size_t)L.num_sms * 4);
-            L.launch(gemm_splitk_finish_kernel<EPI>, dim3(fin), dim3(256), 0, (const float*)L.gemm_ws, splits, p);
-            L.pdl = pdl;
+            L.launch_rows(gemm_splitk_finish_kernel<EPI>, dim3(fin), dim3(256), 0, (const float*)L.gemm_ws, splits, p);
             return;
         }
     }
@@ -135,7 +131,7 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
                 GemmParams full = p;
                 full.tile_begin = 0;
                 full.tile_count = rounds * P;
-                L.launch(gemm_tc_kernel<EPI>, dim3(P), block, tc::SMEM_BYTES, ma, mb, full, error_word);
+                L.launch_rows(gemm_tc_kernel<EPI>, dim3(P), block, tc::SMEM_BYTES, ma, mb, full, error_word);
                 GemmParams q = p;
                 q.tile_begin = rounds * P;
                 q.tile_count = rem;
@@ -147,34 +143,29 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
                     cudaFuncSetAttribute(gemm_tc_kernel<GemmEpi::F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM_BYTES);
                     attr_f32 = true;
                 }
-                L.launch(gemm_tc_kernel<GemmEpi::F32>, dim3(std::min(P, rem * splits)), block, tc::SMEM_BYTES, ma, mb, q, error_word);
+                L.launch_rows(gemm_tc_kernel<GemmEpi::F32>, dim3(std::min(P, rem * splits)), block, tc::SMEM_BYTES, ma, mb, q, error_word);
                 const int per_tile = std::max(1, std::min(32, (P * 4) / rem));
-                L.launch(gemm_tail_finish_kernel<EPI>, dim3(per_tile, rem), dim3(256), 0, (const float*)L.gemm_ws, splits, rounds * P, rem, p);
-                L.pdl = pdl;
+                L.launch_rows(gemm_tail_finish_kernel<EPI>, dim3(per_tile, rem), dim3(256), 0, (const float*)L.gemm_ws, splits, rounds * P, rem, p);
                 return;
             }
         }
     }
-    L.launch(gemm_tc_kernel<EPI>, dim3(std::min(L.num_sms, tiles)), block, tc::SMEM_BYTES, ma, mb, p, error_word);
-    L.pdl = pdl;
+    L.launch_rows(gemm_tc_kernel<EPI>, dim3(std::min(L.num_sms, tiles)), block, tc::SMEM_BYTES, ma, mb, p, error_word);
 }
 
 void launch_gemm_bf16(Launcher& L, const GemmParams& p) { launch_gemm<GemmEpi::Bf16Bias>(L, p); }
 
 void launch_rmsnorm_rows(Launcher& L, const float* x, const __nv_bfloat16* w, __nv_bfloat16* y, int rows, int hidden, float eps) {
-    const bool pdl = L.pdl;
-    L.pdl = pdl && L.pdl_rows;
     // many short rows (vision tower, action model): one warp per row; otherwise one block per row
     if (hidden <= 2048 && (hidden & 3) == 0 && rows >= 256)
-        L.launch(rmsnorm_rows_warp_kernel, dim3((rows + 7) / 8), dim3(256), 0, x, w, y, rows, hidden, eps);
+        L.launch_rows(rmsnorm_rows_warp_kernel, dim3((rows + 7) / 8), dim3(256), 0, x, w, y, rows, hidden, eps);
     else
-        L.launch(rmsnorm_rows_kernel, dim3(rows), dim3(256), 0, x, w, y, hidden, eps);
-    L.pdl = pdl;
+        L.launch_rows(rmsnorm_rows_kernel, dim3(rows), dim3(256), 0, x, w, y, hidden, eps);
 }
 
 void launch_embed_rows(Launcher& L, const int32_t* ids, const __nv_bfloat16* table, const __nv_bfloat16* custom, float* out, int rows,
                        int vocab, int hidden, int embed_token_id, int n_custom, float scale) {
-    L.launch(embed_rows_kernel, dim3(rows), dim3(128), 0, ids, table, custom, out, vocab, hidden, embed_token_id, n_custom, scale);
+    L.launch_rows(embed_rows_kernel, dim3(rows), dim3(128), 0, ids, table, custom, out, vocab, hidden, embed_token_id, n_custom, scale);
 }
 
 void launch_gemm_epi(Launcher& L, GemmEpi epi, const GemmParams& p, int* error_word) {

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <utility>
 #include <vector>
 
 namespace efm {
@@ -13,7 +14,8 @@ namespace efm {
 struct Launcher {
     cudaStream_t stream = nullptr;
     bool pdl = true;                 // programmatic stream serialization between consecutive kernels
-    bool pdl_rows = false;           // keep `pdl` for the row / attention kernels of the prefill family too (they open with the wait)
+    bool rows = false;               // the same for launch_rows: kernels of many-row passes, each of which waits for its predecessor itself
+    bool joined = false;             // the next launch follows another stream's event as well: not programmatic
     int cluster_x = 0;               // next launch only: thread-block cluster of this many blocks along x
     float* gemm_ws = nullptr;        // split-K workspace of the owning context (nullptr: GEMMs never split)
     size_t gemm_ws_floats = 0;
@@ -32,7 +34,7 @@ struct Launcher {
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
         int na = 0;
-        if (pdl) {
+        if (pdl && !joined) {
             attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[na++].val.programmaticStreamSerializationAllowed = 1;
         }
@@ -45,12 +47,23 @@ struct Launcher {
         cfg.attrs = na > 0 ? attr : nullptr;
         cfg.numAttrs = na;
         cluster_x = 0;
+        joined = false;
         err = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
         if (counter != nullptr) ++*counter;
         if (trace != nullptr && err == cudaSuccess) {
             cudaEvent_t ev = nullptr;
             if (cudaEventCreate(&ev) == cudaSuccess) { cudaEventRecord(ev, stream); trace->push_back(ev); }
         }
+    }
+
+    // A kernel that calls pdl_wait() before it touches what its predecessors wrote or read.  Between two such launches of 3 us the GPU
+    // idled 2 to 3 us; started ahead, the next one sets up (barriers, tensor memory, weight tiles) while this one ends.
+    template <typename... KArgs, typename... Args>
+    void launch_rows(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+        const bool keep = pdl;
+        pdl = rows;
+        launch(kernel, grid, block, smem, std::forward<Args>(args)...);
+        pdl = keep;
     }
 };
 

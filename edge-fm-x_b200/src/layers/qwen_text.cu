@@ -403,16 +403,16 @@ void launch_sage_prefill_attention(Launcher& L, const SageScratch& sc, const __n
     L.pdl = false;
     const int kvw = kv_heads * D, qw = q_heads * D;
     const int nkb = (T + kSageBlock - 1) / kSageBlock;
-    L.launch(sage_ksum_kernel, dim3(nkb, kv_heads), dim3(512), 0, k, kvw, T, kv_heads, D, sc.kmean);
+    L.launch_rows(sage_ksum_kernel, dim3(nkb, kv_heads), dim3(512), 0, k, kvw, T, kv_heads, D, sc.kmean);
     const dim3 gk(nkb, kv_heads), gq((S + kSageBlock - 1) / kSageBlock, q_heads);
     if (D == 128) {
-        L.launch(sage_quant_kernel<128>, gk, dim3(512), 0, k, kvw, T, kv_heads, (const float*)sc.kmean, nkb, sc.k8, sc.sk);
-        L.launch(sage_quant_kernel<128>, gq, dim3(512), 0, q, qw, S, q_heads, (const float*)nullptr, 0, sc.q8, sc.sq);
+        L.launch_rows(sage_quant_kernel<128>, gk, dim3(512), 0, k, kvw, T, kv_heads, (const float*)sc.kmean, nkb, sc.k8, sc.sk);
+        L.launch_rows(sage_quant_kernel<128>, gq, dim3(512), 0, q, qw, S, q_heads, (const float*)nullptr, 0, sc.q8, sc.sq);
     } else {
-        L.launch(sage_quant_kernel<64>, gk, dim3(512), 0, k, kvw, T, kv_heads, (const float*)sc.kmean, nkb, sc.k8, sc.sk);
-        L.launch(sage_quant_kernel<64>, gq, dim3(512), 0, q, qw, S, q_heads, (const float*)nullptr, 0, sc.q8, sc.sq);
+        L.launch_rows(sage_quant_kernel<64>, gk, dim3(512), 0, k, kvw, T, kv_heads, (const float*)sc.kmean, nkb, sc.k8, sc.sk);
+        L.launch_rows(sage_quant_kernel<64>, gq, dim3(512), 0, q, qw, S, q_heads, (const float*)nullptr, 0, sc.q8, sc.sq);
     }
-    L.launch(sage_to_half_kernel, dim3(std::min(((size_t)T * kvw / 2 + 255) / 256, (size_t)L.num_sms * 8)), dim3(256), 0, v, kvw, T,
+    L.launch_rows(sage_to_half_kernel, dim3(std::min(((size_t)T * kvw / 2 + 255) / 256, (size_t)L.num_sms * 8)), dim3(256), 0, v, kvw, T,
              kvw, static_cast<__half*>(sc.vh));
     if (D == 128 && attention_tc_enabled()) {
         // tcgen05 form: Qi8 . Ki8^T as kind::i8 into TMEM, P . V in fp16 (attention_tc.cuh, I8 variant)
@@ -434,7 +434,7 @@ void launch_sage_prefill_attention(Launcher& L, const SageScratch& sc, const __n
             a.S = S; a.kv_offset = kv_offset; a.q_heads = q_heads; a.kv_heads = kv_heads; a.kv_rows = T;
             a.scale = 1.0f / sqrtf((float)D);
             a.sq = sc.sq; a.sk = sc.sk; a.error = error;
-            L.launch(seg_attention_tc_kernel<128, true>, dim3((S + at::BM - 1) / at::BM, q_heads), dim3(at::kThreads), C::SMEM, mq, mk, mv, a, error);
+            L.launch_rows(seg_attention_tc_kernel<128, true>, dim3((S + at::BM - 1) / at::BM, q_heads), dim3(at::kThreads), C::SMEM, mq, mk, mv, a, error);
             L.pdl = pdl;
             return;
         }
@@ -461,7 +461,7 @@ void qwen_prefill_chunk(efm_b200_ctx& c, KvSlot& slot, int S, int kv_offset, int
             GemmParams g{c.norm, w.qkv, w.qkv_bias, c.qkv, nullptr, S, QD + 2 * KVD, H};
             launch_gemm_epi(L, GemmEpi::Bf16Bias, g, &c.state->error);
         }
-        L.launch(rope_scatter_kernel, dim3(S), dim3(256), 0,
+        L.launch_rows(rope_scatter_kernel, dim3(S), dim3(256), 0,
                  (const __nv_bfloat16*)c.qkv, c.qbuf, slot.k[l], slot.v[l], (const float*)c.inv_freq,
                  (const int32_t*)c.pos3, S, d.q_heads, d.kv_heads, D, kv_offset, d.use_mrope, d.mrope_section[0],
                  d.mrope_section[0] + d.mrope_section[1]);

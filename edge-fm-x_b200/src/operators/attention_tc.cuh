@@ -165,6 +165,8 @@ __global__ void __launch_bounds__(at::kThreads) seg_attention_tc_kernel(const __
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();          // not before this block has its tensor memory
+    pdl_wait();
     const int kend = s_range[1];
     const int lo_max = s_range[2], hi_min = s_range[3];      // rows past S do not count: their output is never stored
     const int kb0 = s_range[0] == 0x7fffffff ? 0 : (s_range[0] & ~7);          // tile origin: a multiple of 8 keys (TMA alignment)

@@ -57,6 +57,7 @@ template <typename T, bool PRE, bool SUM, bool AVG = false>
 __global__ void __launch_bounds__(256) add_norm_rows_kernel(float* x, const float* x_in, const float* __restrict__ y, const __nv_bfloat16* __restrict__ w,
                                                             T* __restrict__ out, const __nv_bfloat16* __restrict__ pre, int n, int ld, float eps,
                                                             const SumOf<T> sum, const DepthAverage avg) {
+    pdl_enter(x, x_in, y);
     constexpr int KEEP = 4;
     __shared__ float part[2][8];
     const size_t base = (size_t)blockIdx.x * ld;
@@ -201,6 +202,7 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 template <typename T>
 __global__ void __launch_bounds__(256) poly_norm_rows_kernel(const T* __restrict__ z, T* __restrict__ out, const __nv_bfloat16* __restrict__ coef, int n,
                                                              int ld, float eps) {
+    pdl_enter(z);
     constexpr int KEEP = 4;
     __shared__ float part[3][8];
     const size_t base = (size_t)blockIdx.x * ld;
@@ -240,6 +242,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) token_gate_rows_kernel(const float* __restrict__ s, const int32_t* __restrict__ ids,
                                                               const __nv_bfloat16* __restrict__ table, int table_ld, int off, int vocab,
                                                               T* __restrict__ out, int n, int ld) {
+    pdl_enter(s);
     const int row = blockIdx.x, id = ids[row];
     const bool ok = id >= 0 && id < vocab;
     const __nv_bfloat16* e = table + (size_t)(ok ? id : 0) * table_ld + off;
@@ -313,6 +316,7 @@ __global__ void __launch_bounds__(256) relu2_kernel(float* __restrict__ z, size_
 template <typename T>
 __global__ void __launch_bounds__(256) gather_norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows,
                                                                const __nv_bfloat16* __restrict__ w, T* __restrict__ out, int n, int ld, float eps) {
+    pdl_enter(x);
     __shared__ float part[8];
     const float* src = x + (size_t)rows[blockIdx.x] * ld;
     float ss = 0.f;
@@ -334,6 +338,7 @@ struct RowGroups { const int4* tile; const int32_t* n_tiles; int rows; };
 __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int ldw,
                                                        float* __restrict__ C, int ldc, int M, int N, int K, const __nv_bfloat16* __restrict__ bias,
                                                        const RowGroups group) {
+    pdl_enter<false>(A);
     __shared__ float as[16][64 + 4], ws[16][64 + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;

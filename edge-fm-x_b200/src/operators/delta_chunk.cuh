@@ -42,6 +42,7 @@ struct ScanSmem {
 template <int DP>
 __global__ void __launch_bounds__(dc::kThreads) delta_prepare_kernel(const float* __restrict__ proj, const float* __restrict__ decay_in, int ld_decay,
                                                                      float* __restrict__ pack, const DeltaShape s, const RowPlan plan) {
+    pdl_enter<false>(proj, decay_in);
     using namespace dc;
     extern __shared__ __align__(16) unsigned char dc_smem[];
     PrepSmem<DP>& sm = *reinterpret_cast<PrepSmem<DP>*>(dc_smem);
@@ -197,6 +198,7 @@ template <int DP>
 __global__ void __launch_bounds__(dc::kScanThreads) delta_chunk_scan_kernel(const float* __restrict__ pack, float* __restrict__ o, int ld_o,
                                                                         float* __restrict__ pool, size_t slot_stride, size_t offset, const DeltaShape s,
                                                                         const RowPlan plan) {
+    pdl_enter<false>(pack);
     using namespace dc;
     using ds::cp16;
     constexpr int RT = DP / 4;                                     // row tiles of the state (4 x 4 each)

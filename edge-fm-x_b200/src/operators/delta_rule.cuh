@@ -34,6 +34,7 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf
 
 // out[row][0 .. ld_out) = tanh of the last projection segment, zero-padded
 __global__ void __launch_bounds__(128) delta_tanh_rows_kernel(const float* __restrict__ proj, float* __restrict__ out, int ld_out, const DeltaShape s) {
+    pdl_enter<false>(proj);
     const float* src = proj + (size_t)blockIdx.x * s.ld + 5 * s.heads * s.D;
     for (int i = threadIdx.x; i < ld_out; i += 128) out[(size_t)blockIdx.x * ld_out + i] = i < s.rank ? tanhf(src[i]) : 0.f;
 }
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(ds::kThreads) delta_scan_kernel(const float* _
 template <typename TO>
 __global__ void __launch_bounds__(256) delta_output_rows_kernel(const float* __restrict__ o, int ld_o, const float* __restrict__ proj, TO* __restrict__ out,
                                                                 int ld_out, const DeltaShape s, int lanes) {
+    pdl_enter(o, proj);
     const int row = blockIdx.x, HD = s.heads * s.D, l = threadIdx.x & (lanes - 1), per = 256 / lanes;
     const float* orow = o + (size_t)row * ld_o;
     const float* grow = proj + (size_t)row * s.ld + 3 * HD;

@@ -21,6 +21,7 @@ namespace efm {
 
 // one warp per row
 __global__ void __launch_bounds__(256) expert_route_rows_kernel(const float* __restrict__ logits, int ld, int rows, const RouteShape r, const ExpertRows o) {
+    pdl_enter(logits);
     const int row = blockIdx.x * 8 + (int)(threadIdx.x >> 5);
     if (row >= rows) return;
     route_token(logits + (size_t)row * ld, r, [&](int k, int e, float w) {
@@ -56,6 +57,7 @@ __device__ __forceinline__ void expert_offsets(const int32_t* count, int experts
 // Row `row` of h, or (SCALE) each choice's weight times it, to its places in the sorted order.  One block per row; ld % 8 == 0.
 template <typename T, bool SCALE>
 __global__ void __launch_bounds__(128) expert_gather_rows_kernel(const T* __restrict__ h, T* __restrict__ out, int ld, const RouteShape r, const ExpertRows o) {
+    pdl_enter(h);
     __shared__ int32_t off[kMaxExperts];
     __shared__ int32_t dst[kMaxExpertTop];
     __shared__ float weight[SCALE ? kMaxExpertTop : 1];

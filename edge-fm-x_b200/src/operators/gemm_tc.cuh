@@ -211,13 +211,6 @@ __global__ void __launch_bounds__(tc::kThreads) gemm_tc_kernel(const __grid_cons
     volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_m = GROUPED ? *p.group_tiles : (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
-    const int KB_all = (p.K + BK - 1) / BK;
-    const int splits = p.kb_per_split > 0 ? (KB_all + p.kb_per_split - 1) / p.kb_per_split : 1;
-    const int n_tiles = p.tile_count > 0 ? p.tile_count : tiles_m * tiles_n;
-    const int n_items = n_tiles * splits;                             // item = (split, n tile, m tile), m fastest
-    const bool compact = p.tile_count > 0 && p.kb_per_split > 0;      // partial tiles in compact slots
-
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(accf0 + 8 * a, 1); mbar_init(acce0 + 8 * a, kEpiWarps); }
@@ -232,6 +225,15 @@ __global__ void __launch_bounds__(tc::kThreads) gemm_tc_kernel(const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();          // not before this block has its tensor memory: a dependent's block beside it would take it
+    if constexpr (GROUPED) pdl_wait();                                // the tiles are chosen by an earlier kernel
+
+    const int tiles_m = GROUPED ? *p.group_tiles : (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
+    const int KB_all = (p.K + BK - 1) / BK;
+    const int splits = p.kb_per_split > 0 ? (KB_all + p.kb_per_split - 1) / p.kb_per_split : 1;
+    const int n_tiles = p.tile_count > 0 ? p.tile_count : tiles_m * tiles_n;
+    const int n_items = n_tiles * splits;                             // item = (split, n tile, m tile), m fastest
+    const bool compact = p.tile_count > 0 && p.kb_per_split > 0;      // partial tiles in compact slots
 
     auto item_coords = [&](int item, int& m0, int& n0, int& kb0, int& kb1, int& z) {
         if constexpr (GROUPED) {
@@ -255,7 +257,19 @@ __global__ void __launch_bounds__(tc::kThreads) gemm_tc_kernel(const __grid_cons
 
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t it = 0, ahead = 0;
+            if constexpr (!GROUPED) {                                  // B is a weight: the first stages' tiles before the wait
+                if ((int)blockIdx.x < n_items) {
+                    int m0, n0, kb0, kb1, z;
+                    item_coords(blockIdx.x, m0, n0, kb0, kb1, z);
+                    ahead = (uint32_t)min(kb1 - kb0, 2);
+                    for (uint32_t s = 0; s < ahead; ++s) {
+                        mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                        tma_load_2d(base + s * STAGE_BYTES + A_BYTES, &map_b, (kb0 + (int)s) * BK, n0, full0 + 8 * s);
+                    }
+                }
+                pdl_wait();
+            }
             for (int item = blockIdx.x; item < n_items && *abort_s == 0; item += gridDim.x) {
                 int m0, n0, kb0, kb1, z;
                 item_coords(item, m0, n0, kb0, kb1, z);
@@ -264,10 +278,12 @@ __global__ void __launch_bounds__(tc::kThreads) gemm_tc_kernel(const __grid_cons
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1u;
-                    if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, abort_s)) { *abort_s = 1; break; }
-                    mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                    if (it >= ahead) {
+                        if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, abort_s)) { *abort_s = 1; break; }
+                        mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                        tma_load_2d(base + s * STAGE_BYTES + A_BYTES, &map_b, kb * BK, b_row, full0 + 8 * s);
+                    }
                     tma_load_2d(base + s * STAGE_BYTES, &map_a, kb * BK, m0, full0 + 8 * s);
-                    tma_load_2d(base + s * STAGE_BYTES + A_BYTES, &map_b, kb * BK, b_row, full0 + 8 * s);
                 }
             }
         }
@@ -307,6 +323,7 @@ __global__ void __launch_bounds__(tc::kThreads) gemm_tc_kernel(const __grid_cons
         const int q = warp & 3, ch = (warp - 2) >> 2;
         constexpr int LD = 32;
         float* stage = stage_all + (size_t)(warp - 2) * 32 * LD;
+        if constexpr (!GROUPED) pdl_wait();                            // earlier kernels read and write the outputs, too
         int j = 0;
         for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++j) {
             int m0, n0, kb0, kb1, z;
@@ -466,6 +483,7 @@ __global__ void __launch_bounds__(tc::kThreads) gemm_tc_kernel(const __grid_cons
 // partial tiles) -- the order is fixed, so the result does not depend on which block finished first.
 template <GemmEpi EPI>
 __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* __restrict__ ws, int splits, const GemmParams p) {
+    pdl_enter(ws);
     const size_t plane = (size_t)p.M * p.N;
     if constexpr (gemm_is_glu(EPI)) {
         // fused gate|up partials [M, N] (64 gate columns, 64 up columns, ...) -> out [M, N / 2] = unit(gate, up)
@@ -530,6 +548,7 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* __
 template <GemmEpi EPI>
 __global__ void __launch_bounds__(256) gemm_tail_finish_kernel(const float* __restrict__ ws, int splits, int tile_begin, int tile_count,
                                                                const GemmParams p) {
+    pdl_enter(ws);
     constexpr int BM = tc::BM, BN = tc::BN;
     const int tiles_m = (p.M + BM - 1) / BM;
     const int t = blockIdx.y, tile = tile_begin + t;

@@ -49,6 +49,7 @@ constexpr int kLatentRowsPerBlock = 4;
 template <typename T>
 __global__ void __launch_bounds__(32 * kLatentRowsPerBlock) latent_rows_kernel(const T* __restrict__ proj, int ld, T* __restrict__ cq, T* __restrict__ pool,
                                                                                 T* __restrict__ ws, int ws_min_rows, const LatentShape s, const RowPlan plan) {
+    pdl_enter<false>(proj);
     constexpr int KEEP = 6;
     __shared__ float cs_s[kLatentRowsPerBlock][kRotMaxPairs], sn_s[kLatentRowsPerBlock][kRotMaxPairs], rot_s[kLatentRowsPerBlock][2 * kRotMaxPairs];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = blockIdx.x * kLatentRowsPerBlock + warp;
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(32 * kLatentRowsPerBlock) latent_rows_kernel(c
 
 template <typename T>
 __global__ void __launch_bounds__(256) latent_rotate_rows_kernel(T* __restrict__ q, const LatentShape s, const RowPlan plan) {
+    pdl_enter<false>(q);
     __shared__ float cs[kRotMaxPairs], sn[kRotMaxPairs];
     const int row = blockIdx.x, pairs = s.rot.dims / 2;
     const RowEntry e = plan.of_row(row);
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(256) latent_rotate_rows_kernel(T* __restrict__
 template <typename T>
 __global__ void __launch_bounds__(256) latent_gather_rows_kernel(const T* __restrict__ pool, T* __restrict__ ws, int row_elems, const RowPlan plan,
                                                                  const RowTile* __restrict__ pages, int page0) {
+    pdl_enter<false>(pool);
     const RowTile t = pages != nullptr ? pages[blockIdx.x] : RowTile{0, page0 + (int)blockIdx.x};
     const RowEntry e = plan.entry(t.entry);
     const uint4* src = reinterpret_cast<const uint4*>(pool + plan.cache_row(e, t.row * kPageTokens) * row_elems);

@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(256) rope_scatter_kernel(const __nv_bfloat16* 
                                                            const float* __restrict__ inv_freq, const int32_t* __restrict__ pos3,
                                                            int S, int q_heads, int kv_heads, int D, int kv_offset, int use_mrope,
                                                            int sec0, int sec1) {
+    pdl_enter<false>(qkv);
     __shared__ float s_sn[128], s_cs[128];
     const int s = blockIdx.x, half = D >> 1;
     for (int d = threadIdx.x; d < half; d += 256) {

@@ -14,6 +14,7 @@ __global__ void __launch_bounds__(128) embed_rows_kernel(const int32_t* __restri
                                                          const __nv_bfloat16* __restrict__ custom,
                                                          float* __restrict__ out, int vocab, int hidden,
                                                          int embed_token_id, int n_custom, float scale) {
+    pdl_enter(ids, custom);
     const int t = blockIdx.x;
     const int id = ids[t];
     const __nv_bfloat16* src = nullptr;
@@ -35,10 +36,9 @@ __global__ void __launch_bounds__(128) embed_rows_kernel(const int32_t* __restri
 __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* __restrict__ x,
                                                            const __nv_bfloat16* __restrict__ w,
                                                            __nv_bfloat16* __restrict__ y, int hidden, float eps) {
+    pdl_enter(x);
     __shared__ float part[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    pdl_launch_dependents();
-    pdl_wait();            // no-ops unless launched with programmatic stream serialization
     const float* xr = x + (size_t)blockIdx.x * hidden;
     const int nch = hidden >> 3;
     float ss = 0.f;
@@ -74,10 +74,9 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* __restri
 // sum of squares and the scaling (one read of x, no block barrier); 8 rows per block.
 __global__ void __launch_bounds__(256) rmsnorm_rows_warp_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                                 __nv_bfloat16* __restrict__ y, int rows, int hidden, float eps) {
+    pdl_enter(x);
     constexpr int MAXV = 16;                                   // float4 per lane: 16 x 32 x 4 = 2048 channels
     const int row = blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    pdl_launch_dependents();
-    pdl_wait();            // no-ops unless launched with programmatic stream serialization
     if (row >= rows) return;
     const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * hidden);
     const int nv = hidden >> 2;

@@ -25,6 +25,7 @@ constexpr int kSageBlock = 128;      // tokens per quantisation block
 // 512 threads: warp w takes rows w, w + 16, ... (eight independent loads per lane), lane l the channels 4l .. 4l+3.
 __global__ void __launch_bounds__(512) sage_ksum_kernel(const __nv_bfloat16* __restrict__ k, int stride, int T, int heads, int D,
                                                        float* __restrict__ part) {
+    pdl_enter<false>(k);
     __shared__ float red[16][kSageBlock];
     const int b = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = b * kSageBlock;
@@ -60,6 +61,7 @@ template <int D>
 __global__ void __launch_bounds__(512) sage_quant_kernel(const __nv_bfloat16* __restrict__ x, int stride, int T, int heads,
                                                         const float* __restrict__ ksum, int n_part, int8_t* __restrict__ out,
                                                         float* __restrict__ scales) {
+    pdl_enter<false>(x, ksum);
     constexpr int Q = D / 4;                              // elements per thread (32 or 16)
     __shared__ float wmax[16];
     __shared__ float s_scale;
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(512) sage_quant_kernel(const __nv_bfloat16* __
 // bf16 rows [T, heads*D] (row stride `stride`) -> contiguous fp16 [T, heads*D].
 __global__ void __launch_bounds__(256) sage_to_half_kernel(const __nv_bfloat16* __restrict__ x, int stride, int T, int width,
                                                           __half* __restrict__ out) {
+    pdl_enter<false>(x);
     const size_t total = (size_t)T * width / 2;
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {
         const size_t t = (i * 2) / width, c = (i * 2) % width;

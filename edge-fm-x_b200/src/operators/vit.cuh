@@ -12,6 +12,7 @@ namespace efm {
 __global__ void __launch_bounds__(256) vit_gather_blocks_f32_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                                                    const int32_t* __restrict__ order, int n_blocks,
                                                                    int unit, int width) {
+    pdl_enter(src);
     const int per_block = unit * width / 4;
     for (int b = blockIdx.x; b < n_blocks; b += gridDim.x) {
         const float4* s = reinterpret_cast<const float4*>(src + (size_t)order[b] * unit * width);
@@ -24,6 +25,7 @@ __global__ void __launch_bounds__(256) vit_gather_blocks_f32_kernel(const float*
 __global__ void __launch_bounds__(128) vit_scatter_rows_bf16_kernel(const __nv_bfloat16* __restrict__ src,
                                                                    __nv_bfloat16* __restrict__ dst,
                                                                    const int32_t* __restrict__ order, int n_rows, int width) {
+    pdl_enter(src);
     for (int r = blockIdx.x; r < n_rows; r += gridDim.x) {
         const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)r * width);
         uint4* d = reinterpret_cast<uint4*>(dst + (size_t)order[r] * width);
@@ -36,6 +38,7 @@ __global__ void __launch_bounds__(128) vit_scatter_rows_bf16_kernel(const __nv_b
 // inv_freq[i] = theta^(-2 i / (D/2)).  Computed once per encode call.
 __global__ void __launch_bounds__(128) vit_rope_table_kernel(float2* __restrict__ table, const int32_t* __restrict__ pos_h,
                                                             const int32_t* __restrict__ pos_w, int n_patches, int D, float theta) {
+    pdl_enter();
     const int half = D / 2, quarter = D / 4;
     const int i = blockIdx.x * 128 + threadIdx.x;
     if (i >= n_patches * half) return;
@@ -53,6 +56,7 @@ __global__ void __launch_bounds__(128) vit_rope_table_kernel(float2* __restrict_
 // each thread rotates two adjacent pairs of one head (32-bit accesses).
 __global__ void __launch_bounds__(256) vit_rope2d_kernel(__nv_bfloat16* __restrict__ qkv, const float2* __restrict__ table,
                                                         int heads, int D) {
+    pdl_enter<false>(qkv, table);
     const int n = blockIdx.x;
     const int half = D / 2, hp = half / 2;                   // hp: 2-pair groups per head
     __nv_bfloat16* row = qkv + (size_t)n * 3 * heads * D;

@@ -98,6 +98,7 @@ __device__ __forceinline__ void store_head8(T* p, const float (&f)[8]) {        
 template <typename TI, typename TQ, typename TC, bool ROT>
 __global__ void __launch_bounds__(256, 4) qk_scatter_rows_kernel(const TI* __restrict__ qkv, int ld, TQ* __restrict__ q_out, TC* __restrict__ k_pool,
                                                               TC* __restrict__ v_pool, const WindowAttnShape s, const RowPlan plan, int lanes) {
+    pdl_enter<false>(qkv);
     __shared__ __align__(16) float cs[kRotMaxPairs];
     __shared__ __align__(16) float sn[kRotMaxPairs];
     __shared__ float stage[ROT ? 256 * 8 : 1];
@@ -209,6 +210,7 @@ template <typename TQ, typename TC, typename TO>
 __global__ void __launch_bounds__(256) window_attention_rows_kernel(const TQ* __restrict__ q, const TC* __restrict__ k_pool, const TC* __restrict__ v_pool,
                                                                     TO* __restrict__ out, int ld_out, const WindowAttnShape s, const RowPlan plan,
                                                                     const RowTile* __restrict__ tiles) {
+    pdl_enter<false>(q, k_pool, v_pool);
     using namespace wa;
     extern __shared__ __align__(16) float wa_smem[];
     const int tid = threadIdx.x, h = blockIdx.y, g = h / (s.H / s.G);
@@ -685,6 +687,7 @@ template <typename T, int VM>
 __global__ void __launch_bounds__(wd::kThreads) window_attention_short_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool,
                                                                               T* __restrict__ out, int ld_out, const WindowAttnShape s, const RowPlan plan,
                                                                               const int32_t* __restrict__ rows) {
+    pdl_enter<false>(q, k_pool, v_pool);
     using namespace wd;
     constexpr int KC = VM / 32, VK = VM <= 64 ? 4 : (VM <= 128 ? 8 : 16);
     extern __shared__ __align__(16) unsigned char wd_smem[];

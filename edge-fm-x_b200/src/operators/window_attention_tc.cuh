@@ -124,6 +124,8 @@ __global__ void __launch_bounds__(wt::kThreads, 2) window_attention_tc_kernel(co
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();          // not before this block has its tensor memory
+    pdl_wait();
 
     constexpr uint32_t kDescS = instr_desc(BM, BN);
     constexpr uint32_t kDescO = instr_desc(BM, VP) | (1u << 16);
