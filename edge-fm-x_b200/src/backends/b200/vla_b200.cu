@@ -76,6 +76,7 @@ struct efm_b200_vla {
     // vision activations
     __nv_bfloat16 *rows = nullptr, *v_xn = nullptr, *v_qkv = nullptr, *v_attn = nullptr, *v_act = nullptr, *shuf = nullptr;
     float* v_resid = nullptr;
+    float2* rope_tab = nullptr;      // [P + chunk][head_dim / 2] (cos, sin)
     int32_t *v_lo = nullptr, *v_hi = nullptr, *p_lo = nullptr, *p_hi = nullptr, *s_lo = nullptr, *s_hi = nullptr, *c_hi = nullptr;
     // prefix activations
     float* resid = nullptr;
@@ -91,9 +92,7 @@ struct efm_b200_vla {
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t phase_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // set while efm_b200_vla_phase_ms runs
     bool mark_phases = false;
-    bool use_pdl = false;            // EFM_B200_VLA_PDL=1: programmatic dependent launches inside the denoising loop.  Measured on
-                                     // B200: the kernel-by-kernel run gains 15 % (12.2 -> 10.3 ms), the graph replay loses 1.3 %
-                                     // (13.40 -> 13.57 ms per chunk), and the graph is what every call after the first uses
+    bool use_pdl = true;             // dependent launches; EFM_B200_VLA_PDL=0: one launch after the other
 };
 
 namespace {
@@ -276,6 +275,7 @@ efm_status efm_b200_vla_create(const efm_vla_desc* desc, int32_t device, efm_b20
     VTRY(vla_alloc(v, &v->noise, (size_t)(n * d.action_dim)));
     VTRY(vla_alloc(v, &v->x_t, (size_t)(n * d.action_dim)));
     VTRY(vla_alloc(v, &v->time_tab, (size_t)(d.steps * He)));
+    VTRY(vla_alloc(v, &v->rope_tab, (size_t)(v->P + n) * (d.head_dim / 2)));
     VTRY(vla_alloc(v, &v->rows, (size_t)(NV * v->pd)));
     VTRY(vla_alloc(v, &v->v_resid, (size_t)(NV * Hv)));
     VTRY(vla_alloc(v, &v->v_xn, (size_t)(NV * Hv)));
@@ -335,6 +335,12 @@ efm_status efm_b200_vla_create(const efm_vla_desc* desc, int32_t device, efm_b20
             }
         }
         VTRY(cudaMemcpyAsync(v->time_tab, tt.data(), tt.size() * 4, cudaMemcpyHostToDevice, v->stream));
+        const int rope_rows = (int)(v->P + n);
+        Launcher L;
+        L.stream = v->stream;
+        L.pdl = false;
+        L.launch(vla_rope_table_kernel, dim3((rope_rows * (d.head_dim / 2) + 255) / 256), dim3(256), 0, v->rope_tab, rope_rows, d.head_dim, d.rope_theta);
+        VTRY(L.err);
         VTRY(cudaStreamSynchronize(v->stream));
     }
 #undef VTRY
@@ -420,7 +426,7 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
 
     auto mark = [&](int i) { if (v->mark_phases && L.err == cudaSuccess) L.err = cudaEventRecord(v->phase_ev[i], L.stream); };
     mark(0);
-    L.rows = true;
+    L.rows = v->use_pdl;
     // the action state starts as the noise (copied here, far ahead of the loop that launches with programmatic edges)
     if (L.err == cudaSuccess) L.err = cudaMemcpyAsync(v->x_t, v->noise, (size_t)n * d.action_dim * 4, cudaMemcpyDeviceToDevice, L.stream);
     auto layernorm = [&](const __nv_bfloat16* w, const __nv_bfloat16* b) {       // v_resid -> v_xn
@@ -454,7 +460,7 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
     for (LlamaLayer& b : v->vlm) {
         launch_rmsnorm_rows(L, v->resid, b.norm1, v->xn, P, H, d.rms_eps);
         gemm(GemmEpi::Bf16Bias, v->xn, 0, b.qkv_w, nullptr, b.qkv, nullptr, P, QKV, H);
-        L.launch(vla_rope_rows_kernel, dim3(P), dim3(256), 0, b.qkv, QKV, d.q_heads, d.kv_heads, D, 0, d.rope_theta,
+        L.launch_rows(vla_rope_rows_kernel, dim3(P), dim3(256), 0, b.qkv, QKV, d.q_heads, d.kv_heads, D, (const float2*)v->rope_tab,
                  (__nv_bfloat16*)nullptr, 0, 0);
         attend(b.qkv, QKV, b.qkv + QD, b.qkv + QD + KD, QKV, v->attn, P, d.q_heads, d.kv_heads, v->p_lo, v->p_hi);
         gemm(GemmEpi::Residual, v->attn, 0, b.o_w, nullptr, nullptr, v->resid, P, H, QD);
@@ -501,10 +507,9 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
         else if (epi == GemmEpi::Residual) L.launch(skinny_gemm_kernel<SkinnyEpi::Residual, 1>, dim3(N / 8), dim3(kSkinnyThreads), 0, sp);
         else L.launch(skinny_gemm_kernel<SkinnyEpi::Bf16, 1>, dim3(N / 8), dim3(kSkinnyThreads), 0, sp);
     };
-    // the loop's kernels all open with the dependent-launch wait, so they may be launched with programmatic
-    // serialization (off by default, see use_pdl; the tcgen05 GEMM of the chunk > 64 fallback has no such wait)
-    L.pdl = skinny && v->use_pdl;
-    L.rows = L.pdl;
+    // In the loop only the attention is launched ahead of its predecessor's end: it requests the prefix's keys meanwhile.  The products
+    // fill the GPU; placed around their predecessor's blocks they end staggered (all of them ahead: 8.8 ms a chunk against 7.8).
+    L.rows = v->use_pdl;
     for (int s = 0; s < d.steps; ++s) {
         if (skinny) {      // the two wider linears of the suffix embedding on the weight-streaming kernel, bf16 activations
             small(0, v->x_t, d.action_dim, v->ain_w, v->ain_b, v->cat, 2 * He, n, He, d.action_dim, 0.f, v->cat16, 2 * He);
@@ -530,22 +535,23 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
             if (skinny) {          // norm, projection, RoPE and the K / V scatter in one kernel
                 const bool self = l % 2 == 0;
                 SkinnyParams sp{v->e_xn, e.qkv_w, v->e_qkv, nullptr, n, self ? QKV : QD, He, He};
-                sp.q_heads = d.q_heads; sp.kv_heads = self ? d.kv_heads : 0; sp.pos0 = self ? P : 0; sp.theta = d.rope_theta;
+                sp.q_heads = d.q_heads; sp.kv_heads = self ? d.kv_heads : 0; sp.rope = v->rope_tab + (self ? (size_t)P * (D / 2) : 0);
                 sp.kv_out = self ? e.kv : nullptr; sp.kv_stride = 2 * KD; sp.kv_row0 = P; sp.eps = d.rms_eps;
                 L.launch(skinny_gemm_kernel<SkinnyEpi::QkvRope, 2, true>, dim3(sp.N / 16), dim3(kSkinnyThreads), 0, sp);
                 SegAttnParams a{};
                 a.q = v->e_qkv; a.k = e.kv; a.v = e.kv + KD; a.out = v->e_attn; a.lo = v->s_lo; a.hi = self ? v->s_hi : v->c_hi;
                 a.q_stride = self ? QKV : QD; a.kv_stride = 2 * KD; a.out_stride = QD;
                 a.S = n; a.kv_offset = 0; a.q_heads = d.q_heads; a.kv_heads = d.kv_heads; a.scale = scale;
+                a.fixed_rows = P;                                      // the prefix's keys, written before the loop
                 launch_seg_attention_short(L, a, D, self ? P + n : P);
             } else if (l % 2 == 0) {
                 egemm(GemmEpi::Bf16Bias, v->e_xn, e.qkv_w, v->e_qkv, nullptr, QKV, He);
-                L.launch(vla_rope_rows_kernel, dim3(n), dim3(256), 0, v->e_qkv, QKV, d.q_heads, d.kv_heads, D, P, d.rope_theta, e.kv,
+                L.launch(vla_rope_rows_kernel, dim3(n), dim3(256), 0, v->e_qkv, QKV, d.q_heads, d.kv_heads, D, (const float2*)(v->rope_tab + (size_t)P * (D / 2)), e.kv,
                          2 * KD, P);
                 attend(v->e_qkv, QKV, e.kv, e.kv + KD, 2 * KD, v->e_attn, n, d.q_heads, d.kv_heads, v->s_lo, v->s_hi);
             } else {
                 egemm(GemmEpi::Bf16Bias, v->e_xn, e.qkv_w, v->e_qkv, nullptr, QD, He);
-                L.launch(vla_rope_rows_kernel, dim3(n), dim3(256), 0, v->e_qkv, QD, d.q_heads, 0, D, 0, d.rope_theta,
+                L.launch(vla_rope_rows_kernel, dim3(n), dim3(256), 0, v->e_qkv, QD, d.q_heads, 0, D, (const float2*)v->rope_tab,
                          (__nv_bfloat16*)nullptr, 0, 0);
                 attend(v->e_qkv, QD, e.kv, e.kv + KD, 2 * KD, v->e_attn, n, d.q_heads, d.kv_heads, v->s_lo, v->c_hi);
             }
@@ -558,7 +564,6 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
         L.launch(vla_bf16_to_f32_kernel, dim3((n * He + 255) / 256), dim3(256), 0, (const __nv_bfloat16*)v->e_xn, v->hf, n * He);
         small(0, v->hf, He, v->aout_w, v->aout_b, v->x_t, d.action_dim, n, d.action_dim, He, dt);
     }
-    L.pdl = false;
     L.rows = false;
     mark(4);
 }

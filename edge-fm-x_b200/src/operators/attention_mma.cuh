@@ -31,6 +31,8 @@ struct SegAttnParams {
     const float* sq;             // INT8 variant: scale of each 128-token block and head of q [ceil(S / 128), q_heads] ...
     const float* sk;             // ... and of k [ceil(kv_rows / 128), kv_heads]
     int* error;                  // raised (1) when a bounded pipeline wait of the tcgen05 form gives up; may be null
+    int fixed_rows;              // seg_attention_kernel with all keys at once: key rows below this one are older than the launch's
+                                 // predecessor and are requested before the dependency wait
 };
 
 namespace sa {
@@ -82,7 +84,7 @@ template <int D, int NW, int PRE = 0>
 __global__ void __launch_bounds__(NW * 32) seg_attention_kernel(const SegAttnParams p) {
     using namespace sa;
     pdl_launch_dependents();
-    pdl_wait();            // no-ops unless launched with programmatic stream serialization
+    if (PRE == 0) pdl_wait();          // no-op unless launched with programmatic stream serialization
     constexpr int BQ = 16 * NW, kThreads = 32 * NW;
     constexpr int RB = row_bytes<D>();
     constexpr int KS = D / 16;           // k-steps of Q K^T
@@ -119,13 +121,27 @@ __global__ void __launch_bounds__(NW * 32) seg_attention_kernel(const SegAttnPar
     if (i0 < p.S) { lo0 = p.lo != nullptr ? p.lo[i0] : 0; hi0 = p.hi != nullptr ? p.hi[i0] : p.kv_offset + i0 + 1; }
     if (i1 < p.S) { lo1 = p.lo != nullptr ? p.lo[i1] : 0; hi1 = p.hi != nullptr ? p.hi[i1] : p.kv_offset + i1 + 1; }
 
-    load_tile<D, BQ, kThreads>(sq, p.q + (size_t)h * D, p.q_stride, q0, 0, p.S);
     if (PRE > 0) {
-        for (int tl = 0; tl < ntiles; ++tl) {
-            load_tile<D, BKV, kThreads>(sk0 + tl * BKV * RB, kbase, p.kv_stride, kbegin + tl * BKV, kbegin, kend);
-            load_tile<D, BKV, kThreads>(sv0 + tl * BKV * RB, vbase, p.kv_stride, kbegin + tl * BKV, kbegin, kend);
-        }
-    } else if (ntiles > 0) {
+        // rows [from, to) of the block's keys and values, tile after tile (its rows lie RB apart); behind the last one zeros
+        auto load_rows = [&](int from, int to) {
+            constexpr int CH = D / 8;
+            for (int idx = threadIdx.x; idx < (to - from) * CH; idx += kThreads) {
+                const int r = from + idx / CH, ch = idx % CH;
+                const bool in = kbegin + r < kend;
+                const size_t off = (size_t)(in ? kbegin + r : kbegin) * p.kv_stride + ch * 8;
+                cp_async16(sk0 + r * RB + ch * 16, kbase + off, in ? 16 : 0);
+                cp_async16(sv0 + r * RB + ch * 16, vbase + off, in ? 16 : 0);
+            }
+        };
+        const int early = ntiles > 0 ? max(0, min(p.fixed_rows, kend) - kbegin) : 0;
+        load_rows(0, min(early, ntiles * BKV));
+        pdl_wait();
+        load_tile<D, BQ, kThreads>(sq, p.q + (size_t)h * D, p.q_stride, q0, 0, p.S);
+        load_rows(min(early, ntiles * BKV), ntiles * BKV);
+    } else {
+        load_tile<D, BQ, kThreads>(sq, p.q + (size_t)h * D, p.q_stride, q0, 0, p.S);
+    }
+    if (PRE == 0 && ntiles > 0) {
         load_tile<D, BKV, kThreads>(sk0, kbase, p.kv_stride, kbegin, kbegin, kend);
         load_tile<D, BKV, kThreads>(sv0, vbase, p.kv_stride, kbegin, kbegin, kend);
     }

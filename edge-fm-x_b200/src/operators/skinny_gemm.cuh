@@ -10,6 +10,10 @@
 // RMSNorm in front of a product costs nothing extra (NORM variants): the norm weight is folded into W when the
 // weights are loaded, the rows' sums of squares fall out of the activation vectors the warps load anyway, and the
 // 1 / rms factor is applied to the finished 64 x 8 tile.
+// Bound: latency.  A launch of the denoising loop lasts 4 to 8 us, most of it a chain of memory round trips (weights, two or three
+// batches of activations, sums).  Two blocks of 8 warps fit an SM (128 registers a thread: all loads of a batch in flight; at 146 the
+// gate | up product needed two rounds of blocks, 11.7 us instead of 8.3).  The rotation reads a table: with powf and sincosf in its
+// epilogue the q | k | v product took 12.6 us, 4 us more than gate | up, which has 2.5 times its blocks.
 // k-permutation: inside a 32-wide chunk lane t (= lane % 4) owns the 8 consecutive k values 8t .. 8t+7 of
 // its row, for both operands, and feeds them to two k16 MMA steps; a dot product does not care in which
 // order k is visited as long as both operands agree.
@@ -37,10 +41,10 @@ struct SkinnyParams {
     const __nv_bfloat16* bias = nullptr;
     int act = 0, assign = 0;
     // QkvRope (head_dim 64): columns are q heads | k heads | v heads; q and k get the rotate-half RoPE at position
-    // pos0 + row (inverse frequencies theta^(-2i/64)) on the bf16-rounded projections; q goes to C [M, N] in place
+    // of row r, rope[r][i] = (cos, sin) of pair i, on the bf16-rounded projections; q goes to C [M, N] in place
     // of its columns, rotated k and v of row r to kv_out row kv_row0 + r ([.., kv_stride]: k | v) when kv_out is set
-    int q_heads = 0, kv_heads = 0, pos0 = 0;
-    float theta = 0.f;
+    int q_heads = 0, kv_heads = 0;
+    const float2* rope = nullptr;
     __nv_bfloat16* kv_out = nullptr;
     int kv_stride = 0, kv_row0 = 0;
 };
@@ -71,14 +75,13 @@ __global__ void __launch_bounds__(256) fold_norm_weight_kernel(__nv_bfloat16* __
 // the tile 32 columns further in the same head).
 // NWARPS: warps per block (8, or 16 for long K so that a warp's share of the k-chunks fits one batch of requests).
 template <SkinnyEpi EPI, int TILES, bool NORM = false, int NWARPS = 8>
-__global__ void __launch_bounds__(NWARPS * 32) skinny_gemm_kernel(const SkinnyParams p) {
+__global__ void __launch_bounds__(NWARPS * 32, 16 / NWARPS) skinny_gemm_kernel(const SkinnyParams p) {
     constexpr int GROUP = NWARPS / TILES;                  // warps per tile
     constexpr int BATCH = 4;                               // weight vectors requested ahead per warp
     __shared__ float red[NWARPS][64][8];
     __shared__ float ssq[NORM ? NWARPS : 1][64];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     pdl_launch_dependents();
-    pdl_wait();            // no-ops unless launched with programmatic stream serialization
     const int tile = warp / GROUP, j = warp % GROUP;
     // first output column (in W's row numbering) of this warp's tile
     int n0;
@@ -111,17 +114,23 @@ __global__ void __launch_bounds__(NWARPS * 32) skinny_gemm_kernel(const SkinnyPa
         return a;
     };
 
+    const __nv_bfloat16* wrow = p.W + (size_t)(n0 + g) * p.K + 8 * t;
+    uint4 w[BATCH];
+    auto load_w = [&](int c0) {
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            const int k0 = (c0 + i * GROUP) << 5;
+            w[i] = (tile_ok && k0 + 8 * t + 8 <= p.K) ? ld_stream16(wrow + k0) : make_uint4(0u, 0u, 0u, 0u);   // also false past the last chunk
+        }
+    };
+    load_w(j);
+    const __nv_bfloat16* xcol = p.x + 8 * t;
+    pdl_wait();            // no-op unless launched with programmatic stream serialization
+    asm volatile("" : "+l"(xcol)::"memory");                // no activation is loaded ahead of the wait
     if (tile_ok) {
         const int nchunks = (p.K + 31) >> 5;
-        const __nv_bfloat16* wrow = p.W + (size_t)(n0 + g) * p.K + 8 * t;
-        const __nv_bfloat16* xcol = p.x + 8 * t;
         for (int c0 = j; c0 < nchunks; c0 += GROUP * BATCH) {
-            uint4 w[BATCH];
-#pragma unroll
-            for (int i = 0; i < BATCH; ++i) {
-                const int k0 = (c0 + i * GROUP) << 5;
-                w[i] = (k0 + 8 * t + 8 <= p.K) ? ld_stream16(wrow + k0) : make_uint4(0u, 0u, 0u, 0u);   // also false past the last chunk
-            }
+            if (c0 != j) load_w(c0);
             // two chunks at a time: all sixteen activation vectors are requested before the first MMA needs one, so a
             // batch costs two memory round trips instead of one per m-tile (rows >= M and k >= K read as zeros)
 #pragma unroll
@@ -135,8 +144,8 @@ __global__ void __launch_bounds__(NWARPS * 32) skinny_gemm_kernel(const SkinnyPa
 #pragma unroll
                     for (int mt = 0; mt < 4; ++mt) {
                         const int r0 = 16 * mt + g, r1 = r0 + 8;
-                        xa[u][mt] = (kin && r0 < p.M) ? __ldg(reinterpret_cast<const uint4*>(xcol + (size_t)r0 * p.ldx + k0)) : make_uint4(0u, 0u, 0u, 0u);
-                        xb[u][mt] = (kin && r1 < p.M) ? __ldg(reinterpret_cast<const uint4*>(xcol + (size_t)r1 * p.ldx + k0)) : make_uint4(0u, 0u, 0u, 0u);
+                        xa[u][mt] = (kin && r0 < p.M) ? ld_cached(xcol + (size_t)r0 * p.ldx + k0) : make_uint4(0u, 0u, 0u, 0u);
+                        xb[u][mt] = (kin && r1 < p.M) ? ld_cached(xcol + (size_t)r1 * p.ldx + k0) : make_uint4(0u, 0u, 0u, 0u);
                     }
                 }
                 if (NORM) {
@@ -216,10 +225,9 @@ __global__ void __launch_bounds__(NWARPS * 32) skinny_gemm_kernel(const SkinnyPa
         for (int e = 0; e < 4; ++e) {
             const float a = __bfloat162float(__float2bfloat16_rn(x1[e] * inv)), b = __bfloat162float(__float2bfloat16_rn(x2[e] * inv));
             if (rotate) {
-                float sn, cs;
-                sincosf((float)(p.pos0 + row) * powf(p.theta, -(float)(2 * (f0 + e)) / 64.0f), &sn, &cs);
-                o1[e] = a * cs - b * sn;
-                o2[e] = b * cs + a * sn;
+                const float2 r = p.rope[(size_t)row * 32 + f0 + e];
+                o1[e] = a * r.x - b * r.y;
+                o2[e] = b * r.x + a * r.y;
             } else {
                 o1[e] = a;
                 o2[e] = b;

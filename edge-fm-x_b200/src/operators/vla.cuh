@@ -14,8 +14,7 @@ namespace efm {
 // row as in the convolution weight.  One block per patch row.
 __global__ void __launch_bounds__(256) vla_patch_rows_kernel(const float* __restrict__ images, __nv_bfloat16* __restrict__ rows,
                                                             int S, int p) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(images);
     const int side = S / p, patch = blockIdx.x % (side * side), img = blockIdx.x / (side * side);
     const int pr = patch / side, pc = patch % side, pd = 3 * p * p;
     const float* im = images + (size_t)img * 3 * S * S;
@@ -30,8 +29,7 @@ __global__ void __launch_bounds__(256) vla_patch_rows_kernel(const float* __rest
 // value of the residual stream (the patch GEMM then adds onto it).
 __global__ void __launch_bounds__(256) vla_tile_rows_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ dst,
                                                            int period, int width) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter();
     const __nv_bfloat16* s = src + (size_t)(blockIdx.x % period) * width;
     float* d = dst + (size_t)blockIdx.x * width;
     for (int i = threadIdx.x; i < width; i += 256) d[i] = __bfloat162float(s[i]);
@@ -42,8 +40,7 @@ __global__ void __launch_bounds__(256) vla_tile_rows_kernel(const __nv_bfloat16*
 __global__ void __launch_bounds__(256) layernorm_rows_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                             const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                             int width, float eps) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(x);
     __shared__ float red[8];
     __shared__ float stat[2];
     const float* xr = x + (size_t)blockIdx.x * width;
@@ -77,8 +74,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const float* __rest
 __global__ void __launch_bounds__(256) layernorm_rows_warp_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                                  const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                                  int rows, int width, float eps) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(x);
     const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
     const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * width);
@@ -126,8 +122,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_warp_kernel(const float* _
 // One block per output token; d % 8 == 0.
 __global__ void __launch_bounds__(256) vla_pixel_shuffle_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out,
                                                                int side, int s, int d) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(x);
     const int ts = side / s, per = ts * ts;
     const int img = blockIdx.x / per, tok = blockIdx.x % per, R = tok / ts, C = tok % ts;
     const int d8 = d / 8;
@@ -146,8 +141,7 @@ __global__ void __launch_bounds__(256) vla_prefix_rows_kernel(float* __restrict_
                                                              const int32_t* __restrict__ ids, const float* __restrict__ state,
                                                              const __nv_bfloat16* __restrict__ sw, const __nv_bfloat16* __restrict__ sb,
                                                              int n_img_tok, int n_lang, int H, int state_dim, int vocab) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(ids, state);
     const int r = blockIdx.x;
     float* row = resid + (size_t)r * H;
     const float sc = sqrtf((float)H);
@@ -167,24 +161,30 @@ __global__ void __launch_bounds__(256) vla_prefix_rows_kernel(float* __restrict_
     }
 }
 
-// Rotate-half RoPE (inverse frequencies theta^(-2i/D)) on the q and k parts of qkv rows
-// [rows, (q_heads + 2 kv_heads) * D] (q | k | v along the row), row r at position pos0 + r; q in place,
+// table[pos][i] = (cos, sin) of pos * theta^(-2i/D), i < D / 2; once per policy.
+__global__ void __launch_bounds__(256) vla_rope_table_kernel(float2* __restrict__ table, int rows, int D, float theta) {
+    const int i = blockIdx.x * 256 + threadIdx.x, half = D / 2;
+    if (i >= rows * half) return;
+    float sn, cs;
+    sincosf((float)(i / half) * powf(theta, -(float)(2 * (i % half)) / (float)D), &sn, &cs);
+    table[i] = make_float2(cs, sn);
+}
+
+// Rotate-half RoPE on the q and k parts of qkv rows
+// [rows, (q_heads + 2 kv_heads) * D] (q | k | v along the row), row r by rope[r]; q in place,
 // and when kv_out != nullptr the rotated k and the v of row r are written to kv_out row kv_row0 + r
 // ([.., 2 * kv_heads * D]: k | v) instead of in place.  kv_heads == 0: q only.  One block per row.
 __global__ void __launch_bounds__(256) vla_rope_rows_kernel(__nv_bfloat16* __restrict__ qkv, int row_stride, int q_heads, int kv_heads,
-                                                           int D, int pos0, float theta, __nv_bfloat16* __restrict__ kv_out,
+                                                           int D, const float2* __restrict__ rope, __nv_bfloat16* __restrict__ kv_out,
                                                            int kv_out_stride, int kv_row0) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(qkv);
     const int r = blockIdx.x, half = D / 2;
     __nv_bfloat16* row = qkv + (size_t)r * row_stride;
-    const float pos = (float)(pos0 + r);
     const int heads = q_heads + kv_heads;
     for (int i = threadIdx.x; i < heads * half; i += 256) {
         const int h = i / half, f = i % half;
-        const float inv = powf(theta, -(float)(2 * f) / (float)D);
-        float sn, cs;
-        sincosf(pos * inv, &sn, &cs);
+        const float2 cs_sn = rope[(size_t)r * half + f];
+        const float cs = cs_sn.x, sn = cs_sn.y;
         __nv_bfloat16* x = row + (size_t)h * D;
         const float x1 = __bfloat162float(x[f]), x2 = __bfloat162float(x[f + half]);
         const __nv_bfloat16 o1 = __float2bfloat16_rn(x1 * cs - x2 * sn), o2 = __float2bfloat16_rn(x2 * cs + x1 * sn);
@@ -205,8 +205,7 @@ __global__ void __launch_bounds__(256) vla_rope_rows_kernel(__nv_bfloat16* __res
 // dst rows [0, rows) of width w (stride dst_stride) = src rows (stride src_stride); w % 8 == 0, bf16.
 __global__ void __launch_bounds__(128) vla_copy_rows_kernel(const __nv_bfloat16* __restrict__ src, int src_stride,
                                                            __nv_bfloat16* __restrict__ dst, int dst_stride, int w) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(src);
     const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)blockIdx.x * src_stride);
     uint4* d = reinterpret_cast<uint4*>(dst + (size_t)blockIdx.x * dst_stride);
     for (int i = threadIdx.x; i < w / 8; i += 128) d[i] = s[i];
@@ -220,8 +219,7 @@ template <int ACT>
 __global__ void __launch_bounds__(256) vla_small_linear_kernel(const float* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W,
                                                               const __nv_bfloat16* __restrict__ b, float* __restrict__ y, int ldy,
                                                               int M, int N, int K, float euler, __nv_bfloat16* __restrict__ y16, int ldy16) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(x);
     const int lane = threadIdx.x & 31;
     const int o = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (o >= M * N) return;
@@ -243,8 +241,7 @@ __global__ void __launch_bounds__(256) vla_small_linear_kernel(const float* __re
 // cat[m, off + i] = emb[i] for every row m: the time embedding of this step beside the action embedding.
 __global__ void __launch_bounds__(256) vla_fill_time_kernel(float* __restrict__ cat, int ld, int off, const float* __restrict__ emb,
                                                            int width, __nv_bfloat16* __restrict__ cat16) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter();
     float* d = cat + (size_t)blockIdx.x * ld + off;
     for (int i = threadIdx.x; i < width; i += 256) d[i] = emb[i];
     if (cat16 != nullptr) {                 // bf16 copy with the same layout
@@ -255,8 +252,7 @@ __global__ void __launch_bounds__(256) vla_fill_time_kernel(float* __restrict__ 
 
 // y (fp32 rows) = float(x) of bf16 rows -- the final expert norm output for the fp32 output projection.
 __global__ void __launch_bounds__(256) vla_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ y, int n) {
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_enter(x);
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i < n) y[i] = __bfloat162float(x[i]);
 }
