@@ -654,12 +654,17 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
     }
     if (total_want > 0 && logits == nullptr && sampled == nullptr) return fail(c, EFM_ERR_INVALID_ARGUMENT, "logits are wanted but no buffer was given");
     Launcher L = make_launcher(c);
+    auto sampler = [&] {
+        SampleParams s{};
+        s.vocab = c->d.vocab; s.n_part = 0;
+        s.temperature = c->sampling.temperature; s.top_p = c->sampling.top_p; s.seed = c->sampling.seed;
+        s.wbuf = c->wbuf; s.xchg = sample_xchg(c->wbuf, c->d.vocab);
+        return s;
+    };
     auto emit_sample = [&](const float* row, int64_t idx, uint32_t rng_step) -> efm_status {
         if (sampled == nullptr) return (efm_status)EFM_OK;
-        SampleParams s{};
-        s.logits = row; s.vocab = c->d.vocab; s.n_part = 0;
-        s.temperature = c->sampling.temperature; s.top_p = c->sampling.top_p; s.seed = c->sampling.seed; s.rng_step = rng_step;
-        s.token_single = c->tokens_out; s.wbuf = c->wbuf; s.xchg = sample_xchg(c->wbuf, c->d.vocab);
+        SampleParams s = sampler();
+        s.logits = row; s.rng_step = rng_step; s.token_single = c->tokens_out;
         const bool pdl = L.pdl;
         L.pdl = false;
         launch_sample(L, s);
@@ -778,12 +783,29 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
             const int n = (int)std::min(wants.size() - w0, (size_t)m.max_want);
             decoder_rows_logits(*c, m.step_buf + o_want + w0, n, L);
             if (L.err != cudaSuccess) return cuda_fail(c, L.err, "step launch");
-            for (int i = 0; i < n; ++i) {
+            // all rows are sampled before any is copied, and rows that lie together in the caller's buffers travel together: with one
+            // launch and two copies a row, 16 rows cost 0.4 ms of a step of 3.2
+            if (sampled != nullptr) {
+                SampleParams s = sampler();
+                s.logits = m.logits_rows; s.logits_stride = m.head.Np; s.token_single = c->tokens_out;
+                const bool greedy = s.temperature < 1e-6f, pdl = L.pdl;
+                L.pdl = L.rows;
+                if (greedy) launch_sample(L, s, n);
+                for (int i = 0; i < n && !greedy; ++i) {       // the weights of a vocabulary are scratch of one row at a time
+                    s.logits = m.logits_rows + (size_t)i * m.head.Np; s.token_single = c->tokens_out + i; s.rng_step = wants[w0 + i].rng_step;
+                    launch_sample(L, s);
+                }
+                L.pdl = pdl;
+                if (L.err != cudaSuccess) return cuda_fail(c, L.err, "sampler launch");
+            }
+            for (int i = 0, e; i < n; i = e) {
                 const int64_t idx = wants[w0 + i].idx;
-                const float* row = m.logits_rows + (size_t)i * m.head.Np;
-                if (logits != nullptr) EFM_CK(c, cudaMemcpyAsync(logits + (size_t)idx * c->d.vocab, row, (size_t)c->d.vocab * 4, cudaMemcpyDeviceToHost, c->stream));
-                const efm_status ss = emit_sample(row, idx, wants[w0 + i].rng_step);
-                if (ss != EFM_OK) return ss;
+                for (e = i + 1; e < n && wants[w0 + e].idx == idx + (e - i);) ++e;
+                const size_t row = (size_t)c->d.vocab * 4;
+                if (logits != nullptr)
+                    EFM_CK(c, cudaMemcpy2DAsync(logits + (size_t)idx * c->d.vocab, row, m.logits_rows + (size_t)i * m.head.Np, (size_t)m.head.Np * 4, row, (size_t)(e - i),
+                                                cudaMemcpyDeviceToHost, c->stream));
+                if (sampled != nullptr) EFM_CK(c, cudaMemcpyAsync(sampled + idx, c->tokens_out + i, (size_t)(e - i) * 4, cudaMemcpyDeviceToHost, c->stream));
             }
         }
         if (L.err != cudaSuccess) return cuda_fail(c, L.err, "step launch");

@@ -42,11 +42,11 @@ cudaError_t configure_sampler() {
 
 // Greedy decoding needs one block (the arg-max of the logits pass's partial maxima); top-p sampling
 // spreads its passes over the vocabulary across one cluster.
-void launch_sample(Launcher& L, const SampleParams& p) {
+void launch_sample(Launcher& L, const SampleParams& p, int rows) {
     if (g_sampler_cluster < 0) (void)configure_sampler();
     const int cs = (p.temperature >= 1e-6f && p.xchg != nullptr) ? g_sampler_cluster : 1;
     L.cluster_x = cs;
-    L.launch(sample_kernel, dim3(cs), dim3(1024), 0, p);
+    L.launch(sample_kernel, dim3(cs, rows), dim3(1024), 0, p);
 }
 
 // fewest 64-wide k-blocks a split may get (EFM_B200_GEMM_MIN_KB overrides, for measurements)

@@ -20,7 +20,7 @@ bool attention_tc_enabled();
 void launch_seg_attention(Launcher& L, const SegAttnParams& p, int D);
 // Same result; picks the all-keys-resident variant when D == 64, S <= 64 and max_keys (largest hi) <= 320.
 void launch_seg_attention_short(Launcher& L, const SegAttnParams& p, int D, int max_keys);
-void launch_sample(Launcher& L, const SampleParams& p);
+void launch_sample(Launcher& L, const SampleParams& p, int rows = 1);      // rows > 1: greedy, see SampleParams
 cudaError_t configure_sampler();      // once per device at set-up, never inside a stream capture
 // out[r,:] = table[ids[r],:] * scale (fp32), injected rows for ids in [embed_token_id, embed_token_id + n_custom).
 void launch_embed_rows(Launcher& L, const int32_t* ids, const __nv_bfloat16* table, const __nv_bfloat16* custom, float* out, int rows,

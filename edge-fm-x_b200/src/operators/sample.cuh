@@ -39,6 +39,7 @@ struct SampleParams {
     int32_t* tokens_out;     // response buffer, written at state->step
     int max_response;
     int32_t* token_single;   // optional single output
+    int logits_stride;       // greedy, many rows (grid.y): row y reads logits + y * logits_stride and writes token_single[y]
     int advance;             // 1: move kv_len / positions / step on to the next decode step
     uint32_t* wbuf;          // [vocab] scratch: integer weights
     unsigned long long* xchg;  // [1040] scratch of the multi-block form: segment masses [512] | masses before the pick [512] | pick
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const SampleParams p) {
         }
     } else {
         for (int i = tid; i < p.vocab; i += NT) {
-            const float v = p.logits[i];
+            const float v = p.logits[(size_t)blockIdx.y * p.logits_stride + i];
             if (v > bv) { bv = v; bi = i; }
         }
     }
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const SampleParams p) {
     }
 
     if (tid == 0 && blockIdx.x == 0) {
-        if (p.token_single != nullptr) *p.token_single = token;
+        if (p.token_single != nullptr) p.token_single[blockIdx.y] = token;
         if (p.state != nullptr) {
             const int step = p.state->step;
             if (p.tokens_out != nullptr && step >= 0 && step < p.max_response) p.tokens_out[step] = token;
