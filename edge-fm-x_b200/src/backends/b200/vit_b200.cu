@@ -397,13 +397,16 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
     Launcher L;
     L.stream = st;
     L.pdl = false;
-    L.rows = c->pdl;
+    L.rows = c->pdl && tp <= 1;
     L.counter = &c->launches;
     L.gemm_ws = c->gemm_ws;
     L.gemm_ws_floats = c->gemm_ws_floats;
     L.num_sms = c->num_sms;
     int* err = &c->state->error;
-    auto norm_rows = [&](const __nv_bfloat16* w) { if (n > 0) launch_rmsnorm_rows(L, v->resid, w, v->xn, n, H, d.rms_eps); };
+    auto residual = [&](GemmParams g, const __nv_bfloat16* norm) {                       // and the norm behind it
+        g.post_w = norm; g.post_y = v->xn; g.post_eps = d.rms_eps;
+        launch_gemm_epi(L, GemmEpi::Residual, g, err);
+    };
     auto gather_v = [&](const void* send, void* recv, size_t row_bytes, int per) {      // rows cut[r]/per .. cut[r+1]/per of every rank
         size_t off[8], cnt[8];
         for (int r = 0; r < tp; ++r) { off[r] = (size_t)(cut[r] / per) * row_bytes; cnt[r] = (size_t)((cut[r + 1] - cut[r]) / per) * row_bytes; }
@@ -423,11 +426,11 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
     if (n > 0)
         L.launch_rows(vit_rope_table_kernel, dim3((n * (D / 2) + 127) / 128), dim3(128), 0, v->rope_tab, (const int32_t*)(pos_h + r0),
                  (const int32_t*)(pos_w + r0), n, D, d.rope_theta);
+    if (n > 0) launch_rmsnorm_rows(L, v->resid, d.depth > 0 ? v->blocks[0].norm1 : v->ln_q, v->xn, n, H, d.rms_eps);
     for (int l = 0; l < d.depth; ++l) {
         const VitBlock& b = v->blocks[l];
         bool full = false;
         for (int i = 0; i < d.n_fullatt; ++i) full = full || d.fullatt[i] == l;
-        norm_rows(b.norm1);
         if (n > 0) {
             GemmParams g{v->xn, b.qkv_w, b.qkv_b, v->qkv, nullptr, n, 3 * H, H};
             launch_gemm_epi(L, GemmEpi::Bf16Bias, g, err);
@@ -450,19 +453,15 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
             a.kv_rows = full && tp > 1 ? N : n;          // rows behind k / v: the gathered rows of every rank, or the local ones
             a.error = err;
             launch_seg_attention(L, a, D);
-            GemmParams g{v->attn, b.proj_w, b.proj_b, nullptr, v->resid, n, H, H};
-            launch_gemm_epi(L, GemmEpi::Residual, g, err);
+            residual(GemmParams{v->attn, b.proj_w, b.proj_b, nullptr, v->resid, n, H, H}, b.norm2);
         }
-        norm_rows(b.norm2);
         if (n > 0) {
             GemmParams g{v->xn, b.gate_up_w, b.gate_up_b, v->act, nullptr, n, 2 * Ip, H};
             launch_gemm_epi(L, GemmEpi::SwiGlu, g, err);
-            GemmParams g2{v->act, b.down_w, b.down_b, nullptr, v->resid, n, H, Ip};
-            launch_gemm_epi(L, GemmEpi::Residual, g2, err);
+            residual(GemmParams{v->act, b.down_w, b.down_b, nullptr, v->resid, n, H, Ip}, l + 1 < d.depth ? v->blocks[l + 1].norm1 : v->ln_q);
         }
     }
     {   // merger: norm, 4 rows -> one, MLP with exact GELU, back to the original token order
-        norm_rows(v->ln_q);
         if (nm > 0) {
             GemmParams g0{v->xn, v->m0_w, v->m0_b, v->h1, nullptr, nm, v->merged, v->merged};
             launch_gemm_epi(L, GemmEpi::Bf16Gelu, g0, err);

@@ -61,6 +61,14 @@ static bool tail_split_enabled() {
     return on;
 }
 
+// The norm behind a residual product, where no other launch has done it.
+template <GemmEpi EPI>
+static void launch_post_norm(Launcher& L, const GemmParams& p) {
+    if constexpr (EPI == GemmEpi::Residual) {
+        if (p.post_w != nullptr) launch_rmsnorm_rows(L, p.Cf, p.post_w, p.post_y, p.M, p.N, p.post_eps);
+    }
+}
+
 template <GemmEpi EPI>
 static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = nullptr) {
     static bool attr_set = false;
@@ -106,9 +114,17 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
                 attr_f32 = true;
             }
             L.launch_rows(gemm_tc_kernel<GemmEpi::F32>, dim3(std::min(L.num_sms, tiles * splits)), block, tc::SMEM_BYTES, ma, mb, q, error_word);
+            if constexpr (EPI == GemmEpi::Residual) {
+                if (p.post_w != nullptr && p.N <= kFinishNormMax) {
+                    L.launch_rows(p.N <= kFinishNormMax / 4 ? gemm_splitk_finish_norm_kernel<kFinishNormKeep / 4> : gemm_splitk_finish_norm_kernel<kFinishNormKeep>,
+                                  dim3(p.M), dim3(256), 0, (const float*)L.gemm_ws, splits, p);
+                    return;
+                }
+            }
             const size_t total4 = (size_t)p.M * p.N / (gemm_is_glu(EPI) ? 8 : 4);
             const int fin = (int)std::min<size_t>((total4 + 255) / 256, (size_t)L.num_sms * 4);
             L.launch_rows(gemm_splitk_finish_kernel<EPI>, dim3(fin), dim3(256), 0, (const float*)L.gemm_ws, splits, p);
+            launch_post_norm<EPI>(L, p);
             return;
         }
     }
@@ -146,11 +162,13 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
                 L.launch_rows(gemm_tc_kernel<GemmEpi::F32>, dim3(std::min(P, rem * splits)), block, tc::SMEM_BYTES, ma, mb, q, error_word);
                 const int per_tile = std::max(1, std::min(32, (P * 4) / rem));
                 L.launch_rows(gemm_tail_finish_kernel<EPI>, dim3(per_tile, rem), dim3(256), 0, (const float*)L.gemm_ws, splits, rounds * P, rem, p);
+                launch_post_norm<EPI>(L, p);
                 return;
             }
         }
     }
     L.launch_rows(gemm_tc_kernel<EPI>, dim3(std::min(L.num_sms, tiles)), block, tc::SMEM_BYTES, ma, mb, p, error_word);
+    launch_post_norm<EPI>(L, p);
 }
 
 void launch_gemm_bf16(Launcher& L, const GemmParams& p) { launch_gemm<GemmEpi::Bf16Bias>(L, p); }

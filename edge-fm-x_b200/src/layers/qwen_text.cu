@@ -456,7 +456,7 @@ void qwen_prefill_chunk(efm_b200_ctx& c, KvSlot& slot, int S, int kv_offset, int
     launch_embed_rows(L, c.ids, c.embed, n_custom > 0 ? c.custom_embeds : nullptr, c.resid, S, d.vocab, H, embed_token_id, n_custom);
     for (int l = 0; l < d.num_layers; ++l) {
         const LayerWeights& w = c.layers[l];
-        launch_rmsnorm_rows(L, c.resid, w.in_norm, c.norm, S, H, d.rms_eps);
+        if (l == 0 || c.tp_size > 1) launch_rmsnorm_rows(L, c.resid, w.in_norm, c.norm, S, H, d.rms_eps);      // else behind W_down
         {
             GemmParams g{c.norm, w.qkv, w.qkv_bias, c.qkv, nullptr, S, QD + 2 * KVD, H};
             launch_gemm_epi(L, GemmEpi::Bf16Bias, g, &c.state->error);
@@ -471,19 +471,21 @@ void qwen_prefill_chunk(efm_b200_ctx& c, KvSlot& slot, int S, int kv_offset, int
             launch_prefill_attention(L, c.qbuf, slot.k[l], slot.v[l], c.attn, S, kv_offset, d.q_heads, d.kv_heads, D, &c.state->error);
         if (c.tp_size == 1) {
             GemmParams g{c.attn, w.o, nullptr, nullptr, c.resid, S, H, QD};
+            g.post_w = w.post_norm; g.post_y = c.norm; g.post_eps = d.rms_eps;
             launch_gemm_epi(L, GemmEpi::Residual, g, &c.state->error);
         } else {      // row-parallel: this rank's input columns, fp32 partial, all-reduce, then the residual add
             GemmParams g{c.attn + (size_t)c.att_rep_idx * c.o_k, w.o, nullptr, nullptr, c.ybuf, S, H, c.o_k, QD};
             launch_gemm_epi(L, GemmEpi::F32, g, &c.state->error);
             tp_prefill_sum(c, L, S, 0);
         }
-        launch_rmsnorm_rows(L, c.resid, w.post_norm, c.norm, S, H, d.rms_eps);
+        if (c.tp_size > 1) launch_rmsnorm_rows(L, c.resid, w.post_norm, c.norm, S, H, d.rms_eps);
         {     // gate|up with silu(gate) * up in the epilogue
             GemmParams g{c.norm, w.gate_up, nullptr, c.act, nullptr, S, 2 * I, H};
             launch_gemm_epi(L, GemmEpi::SwiGlu, g, &c.state->error);
         }
         if (c.tp_size == 1) {
             GemmParams g{c.act, w.down, nullptr, nullptr, c.resid, S, H, I};
+            if (l + 1 < d.num_layers) { g.post_w = c.layers[l + 1].in_norm; g.post_y = c.norm; g.post_eps = d.rms_eps; }
             launch_gemm_epi(L, GemmEpi::Residual, g, &c.state->error);
         } else {
             GemmParams g{c.act, w.down, nullptr, nullptr, c.ybuf, S, H, I};

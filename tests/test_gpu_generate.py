@@ -47,6 +47,20 @@ def check_against_oracle(cfg, weights, prompt, steps, tokens, logits, **okw):
     return ties
 
 
+@pytest.mark.parametrize("rows", [2, 17, 131])
+@pytest.mark.parametrize("hidden,q_heads,kv_heads,intermediate", [(896, 14, 2, 1024), (1024, 16, 4, 576), (2304, 36, 6, 640), (256, 4, 2, 2048)])
+def test_norm_behind_split_products(rows, hidden, q_heads, kv_heads, intermediate):
+    """A residual product split along K leaves the next norm's rows: one, one full and three parts of 1024 channels, K long enough in both
+    products, in one of them, and another number of rows than a tile has."""
+    cfg = synth.tiny_config(num_layers=2, hidden=hidden, q_heads=q_heads, kv_heads=kv_heads, intermediate=intermediate, vocab=900)
+    w = synth.make_weights(cfg, seed=5)
+    be = make_backend(cfg, w)
+    prompt = synth.make_token_ids(rows + 1, seed=3, vocab=cfg.vocab)
+    toks, logits = cabi.generate(be, 0, prompt, 2, collect_logits=True)
+    check_against_oracle(cfg, w, prompt, 2, toks, logits)
+    be.close()
+
+
 @pytest.mark.parametrize("name,kw,seed", [
     ("qwen2_tiny_tied", dict(num_layers=2, hidden=128, q_heads=2, kv_heads=1, intermediate=256, vocab=1000, tied=True), 0),
     ("qwen2_small_untied", dict(num_layers=3, hidden=256, q_heads=4, kv_heads=2, intermediate=512, vocab=2000,
