@@ -517,6 +517,7 @@ efm_status efm_b200_decoder_create(const efm_decoder_desc* desc, const efm_decod
     m->max_want = std::min(S, 256);
     EFM_TRY(act(&m->head_a, (size_t)m->max_want * Wp));
     EFM_TRY(dev_alloc(c, &m->logits_rows, (size_t)m->max_want * m->head.Np));
+    EFM_TRY(dev_alloc(c, &m->step_tokens, m->max_want));
     // per pass: ids, row entries, wanted rows, short rows, tile and page lists, entries
     m->step_words = (size_t)S * 4 + 2 * (size_t)S * 2 + (size_t)m->ws_pages * 2 + (size_t)S * (sizeof(RowEntry) / 4) + 64;
     EFM_TRY(dev_alloc(c, &m->step_buf, m->step_words));
@@ -537,7 +538,7 @@ efm_status efm_b200_decoder_create(const efm_decoder_desc* desc, const efm_decod
     c->gemm_ws_floats = (size_t)c->num_sms * 128 * 256;
     EFM_TRY(dev_alloc(c, &c->gemm_ws, c->gemm_ws_floats, false));
     EFM_TRY(dev_alloc(c, &c->state, 1));
-    EFM_TRY(dev_alloc(c, &c->tokens_out, (size_t)std::max(desc->max_response_tokens, m->max_want)));
+    EFM_TRY(dev_alloc(c, &c->tokens_out, (size_t)desc->max_response_tokens));
     EFM_TRY(cudaStreamSynchronize(c->stream));
 #undef EFM_TRY
     *out = c;
@@ -664,13 +665,13 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
     auto emit_sample = [&](const float* row, int64_t idx, uint32_t rng_step) -> efm_status {
         if (sampled == nullptr) return (efm_status)EFM_OK;
         SampleParams s = sampler();
-        s.logits = row; s.rng_step = rng_step; s.token_single = c->tokens_out;
+        s.logits = row; s.rng_step = rng_step; s.token_single = m.step_tokens;
         const bool pdl = L.pdl;
         L.pdl = false;
         launch_sample(L, s);
         L.pdl = pdl;
         if (L.err != cudaSuccess) return cuda_fail(c, L.err, "sampler launch");
-        EFM_CK(c, cudaMemcpyAsync(sampled + idx, c->tokens_out, 4, cudaMemcpyDeviceToHost, c->stream));
+        EFM_CK(c, cudaMemcpyAsync(sampled + idx, m.step_tokens, 4, cudaMemcpyDeviceToHost, c->stream));
         return EFM_OK;
     };
     m.tap_row0 = 0;
@@ -787,12 +788,12 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
             // launch and two copies a row, 16 rows cost 0.4 ms of a step of 3.2
             if (sampled != nullptr) {
                 SampleParams s = sampler();
-                s.logits = m.logits_rows; s.logits_stride = m.head.Np; s.token_single = c->tokens_out;
+                s.logits = m.logits_rows; s.logits_stride = m.head.Np; s.token_single = m.step_tokens;
                 const bool greedy = s.temperature < 1e-6f, pdl = L.pdl;
                 L.pdl = L.rows;
                 if (greedy) launch_sample(L, s, n);
                 for (int i = 0; i < n && !greedy; ++i) {       // the weights of a vocabulary are scratch of one row at a time
-                    s.logits = m.logits_rows + (size_t)i * m.head.Np; s.token_single = c->tokens_out + i; s.rng_step = wants[w0 + i].rng_step;
+                    s.logits = m.logits_rows + (size_t)i * m.head.Np; s.token_single = m.step_tokens + i; s.rng_step = wants[w0 + i].rng_step;
                     launch_sample(L, s);
                 }
                 L.pdl = pdl;
@@ -805,7 +806,7 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
                 if (logits != nullptr)
                     EFM_CK(c, cudaMemcpy2DAsync(logits + (size_t)idx * c->d.vocab, row, m.logits_rows + (size_t)i * m.head.Np, (size_t)m.head.Np * 4, row, (size_t)(e - i),
                                                 cudaMemcpyDeviceToHost, c->stream));
-                if (sampled != nullptr) EFM_CK(c, cudaMemcpyAsync(sampled + idx, c->tokens_out + i, (size_t)(e - i) * 4, cudaMemcpyDeviceToHost, c->stream));
+                if (sampled != nullptr) EFM_CK(c, cudaMemcpyAsync(sampled + idx, m.step_tokens + i, (size_t)(e - i) * 4, cudaMemcpyDeviceToHost, c->stream));
             }
         }
         if (L.err != cudaSuccess) return cuda_fail(c, L.err, "step launch");

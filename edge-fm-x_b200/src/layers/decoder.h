@@ -103,6 +103,7 @@ struct DecoderModel {
     // many-row buffers; "act" ones are bf16 or (32-bit mode) fp32
     void *xa = nullptr, *proj_a = nullptr, *q = nullptr, *mix = nullptr, *ff = nullptr, *ff2 = nullptr, *side_a = nullptr, *head_a = nullptr, *cq = nullptr;
     float *y = nullptr, *proj_f = nullptr, *pack = nullptr, *tanh_w = nullptr, *decay = nullptr, *o = nullptr, *side_f = nullptr, *logits_rows = nullptr;
+    int32_t* step_tokens = nullptr;   // [max_want] ids sampled by a batched step (tokens_out belongs to the response that decode steps write)
     int tanh_ld = 0;
     // latent attention, long entries: visible cache rows and what they expand to
     __nv_bfloat16 *ws_c = nullptr, *ws_kv = nullptr;
