@@ -116,7 +116,8 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
             L.launch_rows(gemm_tc_kernel<GemmEpi::F32>, dim3(std::min(L.num_sms, tiles * splits)), block, tc::SMEM_BYTES, ma, mb, q, error_word);
             if constexpr (EPI == GemmEpi::Residual) {
                 if (p.post_w != nullptr && p.N <= kFinishNormMax) {
-                    L.launch_rows(p.N <= kFinishNormMax / 4 ? gemm_splitk_finish_norm_kernel<kFinishNormKeep / 4> : gemm_splitk_finish_norm_kernel<kFinishNormKeep>,
+                    L.launch_rows(rmsnorm_by_warp(p.M, p.N) ? gemm_splitk_finish_norm_kernel<kFinishNormKeep / 4, true>
+                                  : p.N <= kFinishNormMax / 4 ? gemm_splitk_finish_norm_kernel<kFinishNormKeep / 4, false> : gemm_splitk_finish_norm_kernel<kFinishNormKeep, false>,
                                   dim3(p.M), dim3(256), 0, (const float*)L.gemm_ws, splits, p);
                     return;
                 }
@@ -174,8 +175,7 @@ static void launch_gemm(Launcher& L, const GemmParams& p, int* error_word = null
 void launch_gemm_bf16(Launcher& L, const GemmParams& p) { launch_gemm<GemmEpi::Bf16Bias>(L, p); }
 
 void launch_rmsnorm_rows(Launcher& L, const float* x, const __nv_bfloat16* w, __nv_bfloat16* y, int rows, int hidden, float eps) {
-    // many short rows (vision tower, action model): one warp per row; otherwise one block per row
-    if (hidden <= 2048 && (hidden & 3) == 0 && rows >= 256)
+    if (rmsnorm_by_warp(rows, hidden))
         L.launch_rows(rmsnorm_rows_warp_kernel, dim3((rows + 7) / 8), dim3(256), 0, x, w, y, rows, hidden, eps);
     else
         L.launch_rows(rmsnorm_rows_kernel, dim3(rows), dim3(256), 0, x, w, y, hidden, eps);

@@ -549,15 +549,19 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* __
 // The same for a residual product whose rows are normed next: a block per row sums its partials, adds them to the residual and norms
 // the row while it is in registers.  Instead of two launches of 2.4 and 1.6 us at 16 rows (4.6 and 3.3 at 1024), twice a layer: first token
 // of the 0.5B shape 1.85 -> 1.80 ms, a 448 x 448 image 3.01 -> 2.97.
+// The squares of a row are added in the order of the row norm that runs where nothing is split (BY_WARP: rmsnorm_rows_warp_kernel, else
+// rmsnorm_rows_kernel), so that a row's norm does not depend on which of the two computed it: a thread needs other channels than those
+// it summed up, which it reads from shared memory.  448 x 448 image: 2.95 ms in any order, 2.97 in this one (3.03 with every warp reading
+// the row for itself); first token 1.80 both ways, with 40 registers a thread (1.81 with the 48 it would take).
 constexpr int kFinishNormKeep = 8, kFinishNormMax = kFinishNormKeep * 4 * 256;
-template <int KEEP>
-__global__ void __launch_bounds__(256) gemm_splitk_finish_norm_kernel(const float* __restrict__ ws, int splits, const GemmParams p) {
+template <int KEEP, bool BY_WARP>
+__global__ void __launch_bounds__(256, KEEP <= 2 && !BY_WARP ? 6 : 1) gemm_splitk_finish_norm_kernel(const float* __restrict__ ws, int splits, const GemmParams p) {
     pdl_enter(ws);
+    __shared__ float4 sums[KEEP * 256];
     __shared__ float part[8];
     const size_t plane = (size_t)p.M * p.N, row = (size_t)blockIdx.x * p.N;
     const int nv = p.N >> 2, tid = threadIdx.x;                        // N % 4 == 0, at most KEEP * 1024
     float4 x[KEEP];
-    float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < KEEP; ++i) {
         const int c = tid + 256 * i;
@@ -576,14 +580,29 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_norm_kernel(const floa
         }
         x[i] = make_float4(o.x + a.x, o.y + a.y, o.z + a.z, o.w + a.w);
         *reinterpret_cast<float4*>(p.Cf + row + 4 * c) = x[i];
-        ss = fmaf(x[i].x, x[i].x, ss); ss = fmaf(x[i].y, x[i].y, ss); ss = fmaf(x[i].z, x[i].z, ss); ss = fmaf(x[i].w, x[i].w, ss);
+        sums[c] = x[i];
     }
-    ss = warp_sum(ss);
-    if ((tid & 31) == 0) part[tid >> 5] = ss;
     __syncthreads();
     float tot = 0.f;
+    auto square = [&](const float4& v) { tot = fmaf(v.x, v.x, tot); tot = fmaf(v.y, v.y, tot); tot = fmaf(v.z, v.z, tot); tot = fmaf(v.w, v.w, tot); };
+    if constexpr (BY_WARP) {
+        if (tid < 32) {
+#pragma unroll 4
+            for (int c = tid; c < nv; c += 32) square(sums[c]);
+            tot = warp_sum(tot);
+            if (tid == 0) part[0] = tot;
+        }
+        __syncthreads();
+        tot = part[0];
+    } else {
+        for (int c = tid; c < nv >> 1; c += 256) { square(sums[2 * c]); square(sums[2 * c + 1]); }
+        tot = warp_sum(tot);
+        if ((tid & 31) == 0) part[tid >> 5] = tot;
+        __syncthreads();
+        tot = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) tot += part[w];
+        for (int w = 0; w < 8; ++w) tot += part[w];
+    }
     const float inv = 1.0f / sqrtf(tot / (float)p.N + p.post_eps);
 #pragma unroll
     for (int i = 0; i < KEEP; ++i) {

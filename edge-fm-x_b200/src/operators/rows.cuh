@@ -70,6 +70,9 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* __restri
     }
 }
 
+// Many short rows (vision tower, action model): one warp per row; otherwise one block per row.
+__host__ __device__ inline bool rmsnorm_by_warp(int rows, int hidden) { return hidden <= 2048 && (hidden & 3) == 0 && rows >= 256; }
+
 // The same for rows of at most 2048 channels (hidden % 4 == 0): one warp per row, the row stays in registers between the
 // sum of squares and the scaling (one read of x, no block barrier); 8 rows per block.
 __global__ void __launch_bounds__(256) rmsnorm_rows_warp_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ w,

@@ -61,6 +61,37 @@ def test_norm_behind_split_products(rows, hidden, q_heads, kv_heads, intermediat
     be.close()
 
 
+@pytest.mark.parametrize("rows,hidden", [(3, 128), (130, 896), (256, 896), (255, 1024), (300, 2048), (250, 2048), (120, 2304), (256, 2304)])
+def test_norm_behind_a_split_product_is_the_norm_of_its_rows(rows, hidden):
+    """The first layer adds nothing to the stream and both layers take their values to be the normed stream: layer 0 norms its rows by a
+    launch of its own, layer 1 in the sum of W_down's parts.  Every bit agrees; about one value in 40000 did not with the squares added
+    up in another order."""
+    cfg = synth.tiny_config(num_layers=2, hidden=hidden, q_heads=hidden // 64, kv_heads=hidden // 64, intermediate=1024, vocab=700)
+    w = synth.make_weights(cfg, seed=6)
+    w["model.embed_tokens.weight"] *= 50
+    for l in "01":
+        p = f"model.layers.{l}."
+        w[p + "self_attn.v_proj.weight"] = torch.eye(hidden, dtype=torch.bfloat16)
+        w[p + "self_attn.v_proj.bias"].zero_()
+        w[p + "input_layernorm.weight"] = w["model.layers.0.input_layernorm.weight"]
+        w[p + "self_attn.o_proj.weight"].zero_()
+        w[p + "mlp.down_proj.weight"].zero_()
+    be = make_backend(cfg, w, max_tokens=rows, max_prefill_tokens=rows)
+    ids = synth.make_token_ids(rows, seed=3, vocab=cfg.vocab)
+    be.prefill(0, ids, sample=False)
+    be.synchronize()
+    values = []
+    for l in range(2):
+        base, room = be.kv_layer(0, l)
+        holder = type("Layer", (), {"__cuda_array_interface__": dict(shape=(2, room, hidden), typestr="<i2", data=(base, False), version=2)})()
+        values.append(torch.as_tensor(holder, device="cuda").view(torch.bfloat16)[1, :rows].cpu())
+    be.close()
+    x = w["model.embed_tokens.weight"][ids].float()
+    want = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + cfg.rms_eps) * w["model.layers.0.input_layernorm.weight"].float()
+    assert torch.allclose(values[0].float(), want, rtol=2 ** -7, atol=0)       # the values are what they are meant to be: half a bf16 step and the sum's rounding
+    assert torch.equal(values[0].view(torch.int16), values[1].view(torch.int16))
+
+
 @pytest.mark.parametrize("name,kw,seed", [
     ("qwen2_tiny_tied", dict(num_layers=2, hidden=128, q_heads=2, kv_heads=1, intermediate=256, vocab=1000, tied=True), 0),
     ("qwen2_small_untied", dict(num_layers=3, hidden=256, q_heads=4, kv_heads=2, intermediate=512, vocab=2000,
