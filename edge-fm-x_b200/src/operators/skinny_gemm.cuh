@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(NWARPS * 32, 16 / NWARPS) skinny_gemm_kernel(c
             const float a = __bfloat162float(__float2bfloat16_rn(x1[e] * inv)), b = __bfloat162float(__float2bfloat16_rn(x2[e] * inv));
             if (rotate) {
                 const float2 r = p.rope[(size_t)row * 32 + f0 + e];
-                o1[e] = a * r.x - b * r.y;
-                o2[e] = b * r.x + a * r.y;
+                o1[e] = fmaf(a, r.x, -__fmul_rn(b, r.y));
+                o2[e] = fmaf(b, r.x, __fmul_rn(a, r.y));
             } else {
                 o1[e] = a;
                 o2[e] = b;

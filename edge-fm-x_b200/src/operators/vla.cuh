@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(256) vla_rope_table_kernel(float2* __restrict_
 // Rotate-half RoPE on the q and k parts of qkv rows
 // [rows, (q_heads + 2 kv_heads) * D] (q | k | v along the row), row r by rope[r]; q in place,
 // and when kv_out != nullptr the rotated k and the v of row r are written to kv_out row kv_row0 + r
-// ([.., 2 * kv_heads * D]: k | v) instead of in place.  kv_heads == 0: q only.  One block per row.
+// ([.., 2 * kv_heads * D]: k | v) instead of in place.  kv_heads == 0: q only.  One block per row.  Which of a rotation's products is
+// rounded is written out, here and in skinny_gemm.cuh: left to the compiler it changed with the code around it.
 __global__ void __launch_bounds__(256) vla_rope_rows_kernel(__nv_bfloat16* __restrict__ qkv, int row_stride, int q_heads, int kv_heads,
                                                            int D, const float2* __restrict__ rope, __nv_bfloat16* __restrict__ kv_out,
                                                            int kv_out_stride, int kv_row0) {
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(256) vla_rope_rows_kernel(__nv_bfloat16* __res
         const float cs = cs_sn.x, sn = cs_sn.y;
         __nv_bfloat16* x = row + (size_t)h * D;
         const float x1 = __bfloat162float(x[f]), x2 = __bfloat162float(x[f + half]);
-        const __nv_bfloat16 o1 = __float2bfloat16_rn(x1 * cs - x2 * sn), o2 = __float2bfloat16_rn(x2 * cs + x1 * sn);
+        const __nv_bfloat16 o1 = __float2bfloat16_rn(fmaf(x1, cs, -__fmul_rn(x2, sn))), o2 = __float2bfloat16_rn(fmaf(x2, cs, __fmul_rn(x1, sn)));
         if (h >= q_heads && kv_out != nullptr) {
             __nv_bfloat16* d = kv_out + (size_t)(kv_row0 + r) * kv_out_stride + (size_t)(h - q_heads) * D;
             d[f] = o1; d[f + half] = o2;
