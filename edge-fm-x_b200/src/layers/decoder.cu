@@ -230,9 +230,15 @@ void launch_attn_short_v(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, co
     const int hb = (s.H / s.G + wd::kHeads - 1) / wd::kHeads;
     int pages = m.d.cache_pages;
     if (s.window > 0) pages = std::min(pages, (s.window + s.keep + kPageTokens - 1) / kPageTokens);
-    // A block per 64 visible keys, but no more blocks than stay resident at a time (4 a SM): further ones would only add merges.
+    // A block per 64 visible keys, but no wider clusters than are all resident at a time: further ones would only add merges.  How many are
+    // depends on the instance's registers (one or two blocks a SM) and on the width: of 16 blocks fewer fit.  16 rows that see 1040 keys, 16
+    // heads on 4 kv heads, step of 6 layers against four blocks a SM: bf16, 128 channels 492 -> 438 us, 256 channels 1312 -> 912; fp32,
+    // 128 channels 1729 -> 1357.  Wider than resident took up to 75 % more time, except 16 clusters of 256-channel heads that see 4000 keys (17 % less);
+    // half as wide as resident 20 to 70 % more.
+    const int* resident = m.short_resident[VM == 64 ? 0 : VM == 128 ? 1 : 2];
+    const int64_t clusters = (int64_t)s.G * hb * n;
     int splits = 1;
-    while (splits < pages && splits < m.attn_cluster && (int64_t)2 * splits * s.G * hb * n <= 4 * c.num_sms) splits *= 2;
+    for (int w = 1; w < 5 && splits < pages && clusters <= resident[w]; ++w) splits *= 2;
     for (int r0 = 0; r0 < n; r0 += 32768) {                          // grid.z
         L.cluster_x = splits;
         L.launch_rows(window_attention_short_kernel<T, VM>, dim3(splits, s.G * hb, std::min(n - r0, 32768)), dim3(wd::kThreads), sizeof(wd::Smem<VM>),
@@ -1151,9 +1157,31 @@ cudaError_t fit_cluster_v(K kernel, int& width) {
 }
 template <typename TC, int VM, bool ROT>
 cudaError_t fit_cluster(int& width) {
-    cudaError_t e = fit_cluster_v<VM>(window_attention_decode_kernel<TC, VM, ROT, false>, width);
-    if (e == cudaSuccess) e = fit_cluster_v<VM>(window_attention_decode_kernel<TC, VM, ROT, true>, width);
-    return e == cudaSuccess && !ROT ? fit_cluster_v<VM>(window_attention_short_kernel<TC, VM>, width) : e;
+    const cudaError_t e = fit_cluster_v<VM>(window_attention_decode_kernel<TC, VM, ROT, false>, width);
+    return e == cudaSuccess ? fit_cluster_v<VM>(window_attention_decode_kernel<TC, VM, ROT, true>, width) : e;
+}
+// clusters of 1, 2, .. 16 blocks of the kernel for short entries that are resident at a time
+template <typename TC, int VM>
+cudaError_t fit_short(int (&resident)[5]) {
+    const auto kernel = window_attention_short_kernel<TC, VM>;
+    const cudaError_t e = smem_attr(kernel, sizeof(wd::Smem<VM>));
+    if (e != cudaSuccess) return e;
+    const bool wide = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (int w = 0; w < 5; ++w) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1u << w, 1, 1);
+        cfg.blockDim = dim3(wd::kThreads);
+        cfg.dynamicSmemBytes = sizeof(wd::Smem<VM>);
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1u << w;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        if ((w == 4 && !wide) || cudaOccupancyMaxActiveClusters(&resident[w], kernel, &cfg) != cudaSuccess) resident[w] = 0;
+    }
+    (void)cudaGetLastError();
+    return cudaSuccess;
 }
 }  // namespace
 
@@ -1311,6 +1339,9 @@ cudaError_t configure_decoder(DecoderModel& m) {
         if (e == cudaSuccess) e = fit_cluster<TC, 64, true>(m.attn_cluster);
         if (e == cudaSuccess) e = fit_cluster<TC, 128, true>(m.attn_cluster);
         if (e == cudaSuccess) e = fit_cluster<TC, 256, true>(m.attn_cluster);
+        if (e == cudaSuccess) e = fit_short<TC, 64>(m.short_resident[0]);
+        if (e == cudaSuccess) e = fit_short<TC, 128>(m.short_resident[1]);
+        if (e == cudaSuccess) e = fit_short<TC, 256>(m.short_resident[2]);
     };
     if (m.f32) fit(float());
     else fit(__nv_bfloat16());

@@ -134,6 +134,7 @@ struct DecoderModel {
     int32_t* d_route_id = nullptr;
     unsigned int* d_route_ticket = nullptr;
     int attn_cluster = 8, side_cluster = 1;
+    int short_resident[3][5] = {};        // heads of at most 64, 128, 256 channels: clusters of 1, 2, .. 16 blocks of window_attention_short that fit at a time
 };
 
 // One decode step of the bound slot (reads the device state); sample: run the sampler and advance the state.
