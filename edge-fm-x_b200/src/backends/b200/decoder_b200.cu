@@ -519,7 +519,7 @@ efm_status efm_b200_decoder_create(const efm_decoder_desc* desc, const efm_decod
     EFM_TRY(dev_alloc(c, &m->logits_rows, (size_t)m->max_want * m->head.Np));
     EFM_TRY(dev_alloc(c, &m->step_tokens, m->max_want));
     // per pass: ids, row entries, wanted rows, short rows, tile and page lists, entries
-    m->step_words = (size_t)S * 4 + 2 * (size_t)S * 2 + (size_t)m->ws_pages * 2 + (size_t)S * (sizeof(RowEntry) / 4) + 64;
+    m->step_words = (size_t)S * 4 + 3 * (size_t)S * 2 + (size_t)m->ws_pages * 2 + (size_t)S * (sizeof(RowEntry) / 4) + 64;
     EFM_TRY(dev_alloc(c, &m->step_buf, m->step_words));
 
     EFM_TRY(dev_alloc(c, &c->resid_d, Wp));
@@ -703,7 +703,7 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
     while (first < n_entries) {
         std::vector<RowEntry> re;
         std::vector<int32_t> ids, row_entry;
-        std::vector<RowTile> tc, ws;
+        std::vector<RowTile> tc, ws, short_tiles;
         std::vector<int32_t> short_rows;
         int n_ws = 0;
         struct Want { int32_t row; int64_t idx; uint32_t rng_step; };
@@ -715,8 +715,7 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
             KvSlot& s = c->slots.at(en.slot);
             RowEntry r{rows, n, en.kv_offset + done[e], s.table, s.state_slot, 0};
             const int idx = (int)re.size();
-            if (n < kTcMinRows)
-                for (int i = 0; i < n; ++i) short_rows.push_back(rows + i);
+            if (n < kTcMinRows) short_tiles.push_back(RowTile{idx, 0});
             else
                 for (int i = 0; i < n; i += decoder_tc_tile_rows()) tc.push_back(RowTile{idx, i});
             if (n >= kTcMinRows && m.ws_pages > 0) {
@@ -742,6 +741,13 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
         std::vector<RowTile> simt;
         for (size_t i = 0; i < re.size(); ++i)
             for (int r = 0; r < re[i].n && re[i].n >= kTcMinRows; r += decoder_simt_tile_rows()) simt.push_back(RowTile{(int32_t)i, r});
+        RowTiles tiles;
+        tiles.listed = true;
+        std::stable_sort(short_tiles.begin(), short_tiles.end(), [&](const RowTile& a, const RowTile& b) { return re[a.entry].n < re[b.entry].n; });
+        for (const RowTile& t : short_tiles) {
+            for (int r = 0; r < re[t.entry].n; ++r) short_rows.push_back(re[t.entry].row0 + r);
+            ++tiles.short_of[re[t.entry].n];
+        }
         std::vector<int32_t> pk;
         auto put = [&](const void* p, size_t words) {
             const size_t at = pk.size();
@@ -753,7 +759,8 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
         for (const Want& w : wants) want_rows.push_back(w.row);
         const size_t o_ids = put(ids.data(), ids.size()), o_re = put(re.data(), re.size() * sizeof(RowEntry) / 4),
                      o_row = put(row_entry.data(), row_entry.size()), o_tc = put(tc.data(), tc.size() * 2), o_simt = put(simt.data(), simt.size() * 2),
-                     o_want = put(want_rows.data(), want_rows.size()), o_short = put(short_rows.data(), short_rows.size()), o_ws = put(ws.data(), ws.size() * 2);
+                     o_want = put(want_rows.data(), want_rows.size()), o_short = put(short_rows.data(), short_rows.size()), o_ws = put(ws.data(), ws.size() * 2),
+                     o_st = put(short_tiles.data(), short_tiles.size() * 2);
         if (pk.size() > m.step_words) {
             EFM_CK(c, cudaStreamSynchronize(c->stream));
             EFM_CK(c, dev_alloc(c, &m.step_buf, pk.size() * 2, false));
@@ -767,12 +774,11 @@ efm_status efm_b200_decoder_step(efm_b200_ctx* c, const efm_step_entry* entries,
         plan.max_pages = m.d.cache_pages;
         plan.n_entries = (int)re.size();
         plan.rows = rows;
-        RowTiles tiles;
-        tiles.listed = true;
         tiles.tc = reinterpret_cast<const RowTile*>(m.step_buf + o_tc);
         tiles.n_tc = (int)tc.size();
         tiles.simt = reinterpret_cast<const RowTile*>(m.step_buf + o_simt);
         tiles.n_simt = (int)simt.size();
+        tiles.short_tiles = reinterpret_cast<const RowTile*>(m.step_buf + o_st);
         tiles.short_rows = m.step_buf + o_short;
         tiles.n_short = (int)short_rows.size();
         tiles.ws_pages = reinterpret_cast<const RowTile*>(m.step_buf + o_ws);

@@ -246,6 +246,35 @@ void launch_attn_short_v(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, co
                  rows != nullptr ? rows + r0 : nullptr);
     }
 }
+// Short entries of up to how many rows have their rows walked one by one, each by a cluster; the longer ones go to
+// window_attention_rows, a block of 16 rows and one head.  of[n]: entries of n rows.  A row costs its keys once per kv head and block of
+// heads, an entry's block costs them once per head whatever its rows, so few rows in all or heads that share keys favour the first,
+// many rows of many entries the second.  In units of such a block (1.0 us per 700 keys and head of 128 channels on a full chip) a
+// cluster's walk of a row measures a + b x heads of the block: 0.14 + 0.039 x in bf16 (0.17 to 0.18 with one head, 0.43 with eight),
+// 0.10 + 0.037 x, 0.19 + 0.092 x and 0.09 + 0.026 x in fp32 with at most 64, 128 and 256 channels; blocks that do not fill the chip last
+// as long as a full one, two a SM (1.5 with more than 128 channels).  64 entries behind 1500 keys, 8 layers, 8 heads of 128 channels
+// with a kv head each, bf16, rows walked / blocks, ms: 1 row 2.9 / 10.4, 4 rows 9.1 / 10.4, 8 rows 16.8 / 10.5, 15 rows 28 / 10.6.
+template <typename T>
+int short_limit(const WindowAttnShape& s, const int (&of)[kTcMinRows], int num_sms) {
+    const int v = std::max(s.Dp, s.Vp), group = s.H / s.G, hb = (group + wd::kHeads - 1) / wd::kHeads;
+    double a = 0.14, b = 0.039;
+    if (std::is_same<T, float>::value) {
+        a = v <= 64 ? 0.10 : v <= 128 ? 0.19 : 0.09;
+        b = v <= 64 ? 0.037 : v <= 128 ? 0.092 : 0.026;
+    }
+    const double row = (double)s.G * hb * (a + b * std::min(group, wd::kHeads)), full = num_sms * (v <= 128 ? 2.0 : 1.5);
+    int rows = 0, tiles = 0, best = kTcMinRows - 1;
+    for (int n = 1; n < kTcMinRows; ++n) rows += n * of[n];
+    double least = rows * row;
+    for (int n = kTcMinRows - 1; n > 0; --n) {                         // entries of n rows and more in blocks
+        if (of[n] == 0) continue;
+        rows -= n * of[n];
+        tiles += of[n];
+        const double cost = rows * row + std::max(full, (double)tiles * s.H);
+        if (cost < least) { least = cost; best = n - 1; }
+    }
+    return best;
+}
 template <typename T>
 void launch_attn_short(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const DecoderRun& run, const WindowAttnShape& s, const RowPlan& plan, const int32_t* rows, int n) {
     const int v = std::max(s.Dp, s.Vp);
@@ -844,9 +873,21 @@ void attention_rows(efm_b200_ctx& c, Launcher& L, const DecoderLayer& l, const D
             L.launch_rows(window_attention_rows_kernel<TA, TA, TA>, dim3(n, s.H), dim3(256), wa::rows_smem_bytes(s.Dp, s.Vp), static_cast<const TA*>(m.q),
                      (const TA*)kp, (const TA*)vp, static_cast<TA*>(m.mix), l.mix_wp, s, plan, list);
     };
-    if (tiles.listed && tiles.n_short > 0) launch_attn_short<TA>(c, L, l, run, s, plan, tiles.short_rows, tiles.n_short);
+    if (tiles.listed && tiles.n_short > 0) {
+        const int limit = short_limit<TA>(s, tiles.short_of, c.num_sms);
+        int walked = 0, entries = 0, first_tile = 0;
+        for (int n = 1; n < kTcMinRows; ++n) {
+            entries += tiles.short_of[n];
+            if (n <= limit) { walked += n * tiles.short_of[n]; first_tile = entries; }
+        }
+        if (walked > 0) launch_attn_short<TA>(c, L, l, run, s, plan, tiles.short_rows, walked);
+        cuda_cores(tiles.short_tiles + first_tile, entries - first_tile);
+    }
     if (!tiles.listed && plan.rows < kTcMinRows) {
-        launch_attn_short<TA>(c, L, l, run, s, plan, nullptr, plan.rows);
+        int of[kTcMinRows] = {};
+        of[plan.rows] = 1;
+        if (short_limit<TA>(s, of, c.num_sms) >= plan.rows) launch_attn_short<TA>(c, L, l, run, s, plan, nullptr, plan.rows);
+        else cuda_cores(nullptr, 1);
         return;
     }
     if constexpr (std::is_same<TA, __nv_bfloat16>::value) {

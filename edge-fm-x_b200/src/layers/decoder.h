@@ -140,22 +140,25 @@ struct DecoderModel {
 // One decode step of the bound slot (reads the device state); sample: run the sampler and advance the state.
 void decoder_decode_step(efm_b200_ctx& c, KvSlot& slot, Launcher& L, bool sample, bool want_logits);
 // One pass over rows [0, plan.rows) with ids on the device; the residual stream is left in c.resid.
+// Rows of an entry from which on its tiles go to the tensor-core form (layers it takes); shorter entries: see short_limit.
+constexpr int kTcMinRows = 16;
 // Attention work lists of a batched pass (listed): tensor-core tiles of the long entries, the same rows in CUDA-core tiles (layers
-// the tensor-core form does not take), and the rows of the short entries.  Not listed: the single entry.
+// the tensor-core form does not take), and the short entries, fewest rows first: their rows, their CUDA-core tiles (one each) and how
+// many have 1, 2, .. rows.  Not listed: the single entry.
 struct RowTiles {
-    const RowTile *tc = nullptr, *simt = nullptr;
+    const RowTile *tc = nullptr, *simt = nullptr, *short_tiles = nullptr;
     int n_tc = 0, n_simt = 0;
-    // latent attention: workspace pages of the long entries and those of them that hold earlier tokens (listed, or from ws_page0 on)
     const int32_t* short_rows = nullptr;
+    int n_short = 0, short_of[kTcMinRows] = {};
+    // latent attention: workspace pages of the long entries and those of them that hold earlier tokens (listed, or from ws_page0 on)
     const RowTile* ws_pages = nullptr;
-    int n_short = 0, n_ws = 0, n_gather = 0, ws_page0 = 0;
+    int n_ws = 0, n_gather = 0, ws_page0 = 0;
     bool listed = false;
 };
 void decoder_rows_pass(efm_b200_ctx& c, const RowPlan& plan, const int32_t* ids, const RowTiles& tiles, Launcher& L);
 // logits_rows[i] = head . norm(resid[rows[i]]), i < n <= max_want; rows on the device
 void decoder_rows_logits(efm_b200_ctx& c, const int32_t* rows, int n, Launcher& L);
-// Rows of one entry that share an attention block; rows of entries shorter than kTcMinRows are walked one by one.
-constexpr int kTcMinRows = 16;
+// Rows of one entry that share an attention block.
 int decoder_tc_tile_rows();
 int decoder_simt_tile_rows();
 bool decoder_layer_tc(const DecoderModel& m, const DecoderLayer& l);

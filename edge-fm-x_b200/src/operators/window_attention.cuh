@@ -7,9 +7,10 @@
 // Dp / Vp (multiples of 64); a sequence's pages are listed in a page table.  TC = bf16 or fp32 (the all-32-bit mode).
 //
 //   qk_scatter_rows      many rows: per-head norms and rotation, q -> [T][H][Dp], k and v -> cache rows
-//   window_attention_rows many rows on the CUDA cores, fp32 throughout (32-bit mode, head sizes the tensor-core form does not take)
+//   window_attention_rows many rows on the CUDA cores, fp32 throughout (32-bit mode, head sizes the tensor-core form does not take,
+//                        many rows of many short entries)
 //   window_attention_short rows of entries too short for the tensor-core form (decoded tokens of many sequences, short portions):
-//                        the walk of window_attention_decode for every row
+//                        the walk of window_attention_decode for every row, where the rows are few (short_limit in decoder.cu)
 //   window_attention_decode one row: norms of q and k, cache append and split-key attention in one launch; the splits of
 //                        a kv head are the blocks of one cluster and merge through distributed shared memory
 #pragma once

@@ -6,6 +6,7 @@ import pytest
 
 import cabi
 import temuvik_util as tu
+from oracle import temuvik
 from temuvik_util import attention, config, latent
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +56,38 @@ def test_a_step_leaves_the_response_of_a_decoding_slot_alone(built, live, temper
         step(d, [(s, 0, tu.tokens(cfg, 9, seed=s), [], 0)])
     assert response(lambda: step(d, [(s, 9, [s % 150], [0], s) for s in range(live)])) == expected
     d.close()
+
+
+# heads and kv heads: a row walked by a cluster of its own costs least with few kv heads, a block for all rows of an entry with many
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("dim,vdim", [(24, 40), (128, 72), (200, 144)])
+@pytest.mark.parametrize("heads,kv_heads,sizes", [(8, 8, [15]), (8, 8, [15] * 40), (8, 8, [1, 15] * 30), (9, 9, list(range(1, 16)) * 4), (9, 3, [2, 3, 5, 14] * 16),
+                                                  (9, 1, [9, 15] * 24), (8, 8, [5] * 64), (8, 8, [1] * 40 + [16, 33, 7])])
+def test_short_entries_of_any_size(built, heads, kv_heads, sizes, dim, vdim, dtype):
+    """Rows walked one by one, blocks of an entry's rows, and both in one pass, beside entries long enough for the tensor cores; every row
+    against the CPU statement."""
+    cfg = config([attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=0.1, size=70, keep=3), attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, scale=0.1, size=None)],
+                 width=64, vocab=60)
+    w = tu.weights(cfg, seed=8)
+    before = [(7 * i + 61) % 130 + 1 for i in range(len(sizes))]
+    seq = tu.tokens(cfg, 130 + max(sizes))
+    ref = temuvik.forward(cfg, w, seq).logits.numpy()
+    d = decoder(cfg, w, len(sizes), 3, dtype=cabi.EFM_F32 if dtype == "fp32" else cabi.EFM_BF16)
+    step(d, [(s, 0, seq[:n], [], 0) for s, n in enumerate(before)], logits=False, sampled=False)
+    got, _ = step(d, [(s, n, seq[n:n + k], list(range(k)), 0) for s, (n, k) in enumerate(zip(before, sizes))], sampled=False)
+    d.close()
+    assert tu.error(got, np.concatenate([ref[n:n + k] for n, k in zip(before, sizes)])) < tu.LIMIT[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("heads", [8, 120])
+def test_short_prompt_of_many_heads(built, heads, dtype):
+    """The 15 rows in front of a prompt's last token: walked one by one with 8 heads, blocks of all of them with 120."""
+    cfg = config([attention(heads=heads, kv_heads=heads, dim=16, vdim=24, scale=0.1, rot=16, size=10, keep=2)] * 2, width=64, vocab=60)
+    w = tu.weights(cfg, seed=8)
+    seq = tu.tokens(cfg, 16)
+    d = decoder(cfg, w, 1, 1, dtype=cabi.EFM_F32 if dtype == "fp32" else cabi.EFM_BF16)
+    d.prefill(0, seq, sample=True)
+    got = np.array(d.read_logits())
+    d.close()
+    assert tu.error(got[None], temuvik.forward(cfg, w, seq).logits.numpy()[-1:]) < tu.LIMIT[dtype]
