@@ -397,7 +397,7 @@ efm_status efm_b200_vit_encode(efm_b200_vit* v, const void* pixels, int32_t pixe
     Launcher L;
     L.stream = st;
     L.pdl = false;
-    L.rows = c->pdl && tp <= 1;
+    L.rows = c->pdl && tp <= 1;      // ranks exchange rows with collectives between the kernels: in order there, as the text tower's
     L.counter = &c->launches;
     L.gemm_ws = c->gemm_ws;
     L.gemm_ws_floats = c->gemm_ws_floats;

@@ -507,8 +507,10 @@ void vla_forward(efm_b200_vla* v, Launcher& L) {
         else if (epi == GemmEpi::Residual) L.launch(skinny_gemm_kernel<SkinnyEpi::Residual, 1>, dim3(N / 8), dim3(kSkinnyThreads), 0, sp);
         else L.launch(skinny_gemm_kernel<SkinnyEpi::Bf16, 1>, dim3(N / 8), dim3(kSkinnyThreads), 0, sp);
     };
-    // In the loop only the attention is launched ahead of its predecessor's end: it requests the prefix's keys meanwhile.  The products
-    // fill the GPU; placed around their predecessor's blocks they end staggered (all of them ahead: 8.8 ms a chunk against 7.8).
+    // At most 64 rows: the attention is launched ahead of its predecessor's end and requests the prefix's keys meanwhile (8.4 ms a chunk of
+    // 50 without, 7.8 with), and so is the final norm; the products are launched in order.  They fill the GPU; placed around their predecessor's
+    // blocks they end staggered (all of them ahead: 8.8).  More rows: the tcgen05 products, their sums, the norms and the attention are all
+    // launched ahead (65 rows 12.9 -> 11.3 ms, 128 rows 13.7 -> 12.4); the rotation is not.
     L.rows = v->use_pdl;
     for (int s = 0; s < d.steps; ++s) {
         if (skinny) {      // the two wider linears of the suffix embedding on the weight-streaming kernel, bf16 activations

@@ -56,7 +56,9 @@ struct Launcher {
         }
     }
 
-    // A kernel that calls pdl_wait() before it touches what its predecessors wrote or read.  Between two such launches of 3 us the GPU
+    // A kernel that calls pdl_wait() before it touches what its predecessors wrote or read.  Launched in order by launch(), not measured
+    // otherwise: the windowed and the latent attention of layered decoders, their linear attention, input convolutions, rotation tables and
+    // elementwise norms, and the LayerNorm, patch, prefix and copy rows of the action model; a wait in those is a no-op.  Between two such launches of 3 us the GPU
     // idled 2 to 3 us; started ahead, the next one sets up (barriers, tensor memory, weight tiles) while this one ends.
     template <typename... KArgs, typename... Args>
     void launch_rows(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {

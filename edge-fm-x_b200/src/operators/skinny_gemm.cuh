@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 16 / NWARPS) skinny_gemm_kernel(c
     };
     load_w(j);
     const __nv_bfloat16* xcol = p.x + 8 * t;
-    pdl_wait();            // no-op unless launched with programmatic stream serialization
+    pdl_wait();            // a no-op as the action loop launches these products, in order: launched ahead they cost it 1 ms
     asm volatile("" : "+l"(xcol)::"memory");                // no activation is loaded ahead of the wait
     if (tile_ok) {
         const int nchunks = (p.K + 31) >> 5;
