@@ -91,3 +91,55 @@ def test_short_prompt_of_many_heads(built, heads, dtype):
     got = np.array(d.read_logits())
     d.close()
     assert tu.error(got[None], temuvik.forward(cfg, w, seq).logits.numpy()[-1:]) < tu.LIMIT[dtype]
+
+
+LENGTHS = [200, 130, 9, 1]
+
+
+def wants(count):
+    """`count` of the rows of four entries: an entry's last rows in descending order, then rows with gaps, a repeated one, a single one."""
+    lists = [list(range(199, -1, -1)), list(range(1, 130, 2)) + list(range(0, 130, 2)), [8, 8, 0], [0]]
+    share = [max(0, min(len(l), n)) for l, n in zip(lists, (count - 6 - (count - 6) // 3, (count - 6) // 3, 3, 1))] if count > 8 else [0, 0, 0, 1] if count == 1 else [0, count - 1, 0, 1]
+    share[0] += count - sum(share)
+    return [l[:n] for l, n in zip(lists, share)]
+
+
+@pytest.mark.parametrize("max_step_tokens", [2048, 96])
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("vocab", [64, 147])
+@pytest.mark.parametrize("count", [1, 2, 40, 256, 257, 300])
+def test_wanted_rows_of_a_step(built, count, vocab, dtype, max_step_tokens):
+    """Logits and samples of one call, in one pass and in passes that cut entries, up to more rows than the head takes at a time."""
+    cfg = config([attention(), latent()], vocab=vocab)
+    w = tu.weights(cfg, seed=5)
+    seqs = [tu.tokens(cfg, n, seed=n) for n in LENGTHS]
+    d = decoder(cfg, w, 4, 4, max_step_tokens=max_step_tokens, dtype=cabi.EFM_F32 if dtype == "fp32" else cabi.EFM_BF16)
+    lists = wants(count)
+    assert sum(map(len, lists)) == count
+    entries = [(s, 0, seq, l, 0) for s, (seq, l) in enumerate(zip(seqs, lists))]
+    z, ids = step(d, entries)
+    ref = np.concatenate([temuvik.forward(cfg, w, seq).logits.numpy()[l] for seq, l in zip(seqs, lists) if l])
+    assert tu.error(z, ref) < tu.LIMIT[dtype]
+    assert ids.tolist() == z.argmax(1).tolist()
+    assert np.array_equal(step(d, entries, sampled=False)[0], z)
+    assert np.array_equal(step(d, entries, logits=False)[1], ids)
+    d.close()
+
+
+def test_sampled_rows_of_a_step_are_those_of_single_rows(built):
+    """Nucleus samples of many rows in one call, and of the same rows wanted one at a time, with the same counters (32-bit mode: a row's logits do
+    not depend on the others)."""
+    cfg = config([attention(), latent()], vocab=147)
+    w = tu.weights(cfg, seed=5)
+    seqs = [tu.tokens(cfg, n, seed=n) for n in LENGTHS]
+    d = decoder(cfg, w, 4, 4, dtype=cabi.EFM_F32)
+    d.set_sampling(1.2, 0.9, 11)
+    lists = [[199, 4, 77], [0, 1, 2, 129], [8, 8, 3], [0]]
+
+    def entries(lists):
+        return [(s, 0, seq, l, 100 + s) for s, (seq, l) in enumerate(zip(seqs, lists))]
+    z, ids = step(d, entries(lists))
+    alone = [step(d, entries([[p] if t == s else [] for t in range(4)]), logits=False)[1][0] for s, l in enumerate(lists) for p in l]
+    d.close()
+    assert ids.tolist() == alone
+    assert ids.tolist() != z.argmax(1).tolist()
